@@ -18,6 +18,7 @@
 #include "cbm_kernels.cuh"
 #include "cbm_small.cuh"
 #include "cbm_stencil_tma.cuh"
+#include "cbm_tile.cuh"
 #include <utility>
 
 using namespace cbm;
@@ -98,6 +99,7 @@ struct cbm_ctx {
   int n_blocks = 0;
   int n_sm = 148;             // multiprocessors of the device (grid of the compaction)
   int de_blocks = 1;          // persistent grid of the force kernel
+  int tile_blocks = 0;        // resident blocks of k_agent_de_tile (0: not used)
   void* pair_list = nullptr;  // its partner lists (cell walks only)
   void* pos32 = nullptr;      // Float64 3D cell walks: positions rounded to Float32
   void* pos_rows = nullptr;   // Float32 3D cell walks: positions as rows x | y | z
@@ -343,6 +345,7 @@ Params<T> params(const cbm_ctx* c, int parity) {
   P.cut2 = bound2<T>(k.r_rep > k.r_att ? k.r_rep : k.r_att);
   P.skin2 = bound2<T>(k.skin);
   P.skin2_lo = bound2_lo<T>(k.skin);
+  P.tiled = c->tile_blocks > 0;
   P.force_in_list = (T)(k.r_rep > k.r_att ? k.r_rep : k.r_att) <= (T)k.skin ? 1 : 0;
   P.cut_reach = (T)((k.r_rep > k.r_att ? k.r_rep : k.r_att) * (1.0 + 1e-4));
   P.skin_reach = (T)(k.skin * (1.0 + 1e-4));
@@ -374,6 +377,26 @@ bool rule_needed(const cbm_config& k) {
 }
 // the atomic rule path reads the committed field from a snapshot
 bool needs_snapshot(const cbm_config& k) { return k.uptake != 0 && exchanges(k) && !uses_gather(k); }
+
+double cutoff(const cbm_config& k) { return k.r_rep > k.r_att ? k.r_rep : k.r_att; }
+
+// The 3D cell walks that k_agent_de_tile takes: of the committed positions
+// (no wall reflection and no stage positions, whose agents may lie outside
+// the cells they are filed in), with CellLinked, or with CLVD in the steps
+// with births or deaths.
+bool walk_by_tile(const cbm_config& k) {
+  return k.dims == 3 && k.walls != CBM_WALLS_REFLECT &&
+         (k.integrator == CBM_INT_EULER || k.integrator == CBM_INT_EM) &&
+         cutoff(k) <= kTileMaxCutoff &&
+         (k.neighbors == CBM_NEIGH_CELL_LINKED ||
+          (k.neighbors == CBM_NEIGH_CLVD && k.fate != CBM_FATE_NONE));
+}
+// the 3D force-only walks left to k_agent_de, one thread an agent
+bool walk_by_thread(const cbm_config& k) {
+  return k.dims == 3 && !walk_by_tile(k) &&
+         (k.neighbors == CBM_NEIGH_CELL_LINKED ||
+          (k.neighbors == CBM_NEIGH_CLVD && k.fate != CBM_FATE_NONE));
+}
 
 // blocks of the 2D shared-memory stencils (one tile per block)
 dim3 stencil_grid(const cbm_ctx* c) {
@@ -512,8 +535,15 @@ void enqueue_agent_de(cbm_ctx* c, const Params<T>& P) {
     k_pos_rows<T><<<c->n_blocks, kTile, 0, c->stream>>>(P);
   }
   if (integ != CBM_INT_HEUN && integ != CBM_INT_RK4 && integ != CBM_INT_EULER_HEUN) {
+    if constexpr (D == 3) {
+      if (P.tiled) {
+        PROF("k_agent_de_tile");
+        k_agent_de_tile<T><<<c->tile_blocks, 32, 0, c->stream>>>(P);
+      }
+      if (P.tiled && c->cfg.neighbors == CBM_NEIGH_CELL_LINKED) return;
+    }
     PROF("k_agent_de");
-    k_agent_de<T, D><<<grid, kTile, 0, c->stream>>>(P);
+    launch_pdl(c, P.tiled != 0, k_agent_de<T, D>, dim3(grid), dim3(kTile), 0, P);
     return;
   }
   // multi-stage: f at u, then at each stage's positions (own cell from the
@@ -615,6 +645,7 @@ int kernels_per_step(const cbm_ctx* c) {
   if (rule_needed(k)) n += 1;           // rule (with births and deaths when fate is on)
   if (k.fate != CBM_FATE_NONE) n += 1;  // compaction
   n += 1;                               // agent DE
+  if (c->tile_blocks && k.neighbors == CBM_NEIGH_CLVD) n += 1;  // its steps on the list
   if (c->pos32) n += 1;                 // its Float32 positions (Float64 3D walks)
   if (c->pos_rows) n += 1;              // its position rows (Float32 3D walks)
   if (k.medium) n += 1;
@@ -697,6 +728,19 @@ template <typename T, int D>
 struct DEOccupancy {
   static void run(cbm_ctx*, int* bps) {
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_agent_de<T, D>, kTile, 0) !=
+            cudaSuccess ||
+        *bps < 1)
+      *bps = 1;
+  }
+};
+
+// resident one-warp blocks of the tiled force walk per multiprocessor
+template <typename T, int D>
+struct TileOccupancy {
+  static void run(cbm_ctx*, int* bps) {
+    cudaFuncSetAttribute(k_agent_de_tile<T>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                         kTileCarveout);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_agent_de_tile<T>, 32, 0) !=
             cudaSuccess ||
         *bps < 1)
       *bps = 1;
@@ -1052,10 +1096,18 @@ int cbm_create(cbm_ctx** out, const cbm_config* cfg) {
     dispatch<DEOccupancy>(c, &bps);
     const long long resident = (long long)c->n_sm * bps;
     c->de_blocks = (int)(resident < c->n_blocks ? resident : c->n_blocks);
-    if (cells && k.dims == 3)
+    if (walk_by_tile(k)) {
+      dispatch<TileOccupancy>(c, &bps);
+      const long long tiles = (long long)(n + 31) / 32, warps = (long long)c->n_sm * bps;
+      c->tile_blocks = (int)(warps < tiles ? warps : tiles);
+    }
+    if (walk_by_thread(k))
       c->pair_list = dalloc(c, (size_t)c->de_blocks * kTile * kPairCap4 * sizeof(int4), &ok);
-    if (cells && k.dims == 3 && c->tsize == 8) c->pos32 = dalloc(c, n * sizeof(float4), &ok);
-    if (cells && k.dims == 3 && c->tsize == 4) {
+    // the filter's copies of the committed positions (a walk of reflected
+    // positions reads those)
+    const bool copies = walk_by_thread(k) && k.walls != CBM_WALLS_REFLECT;
+    if (copies && c->tsize == 8) c->pos32 = dalloc(c, n * sizeof(float4), &ok);
+    if (copies && c->tsize == 4) {
       c->rows_stride = (int)((n + 3) & ~(size_t)3);  // rows start on 16 bytes
       c->pos_rows = dalloc(c, 3 * (size_t)c->rows_stride * sizeof(float), &ok);
     }

@@ -63,6 +63,7 @@ struct Params {
   const V4* XS;
   V4* KOUT;
   int no_prune;
+  int tiled;            // k_agent_de_tile takes the 3D cell walks of this configuration
   V4* POLD;             // positions at the last Verlet rebuild (slot order)
   int* inv;             // agent index -> slot of A
   int* cell_of_slot;    // cell of each A slot
@@ -1084,6 +1085,15 @@ __device__ __forceinline__ float2 f2_mul(float2 a, float2 b) {
   return *reinterpret_cast<float2*>(&r);
 }
 
+__device__ __forceinline__ float2 f2_add(float2 a, float2 b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(r)
+      : "l"(*reinterpret_cast<unsigned long long*>(&a)),
+        "l"(*reinterpret_cast<unsigned long long*>(&b)));
+  return *reinterpret_cast<float2*>(&r);
+}
+
 __device__ __forceinline__ float2 f2_fma(float2 a, float2 b, float2 c) {
   unsigned long long r;
   asm("fma.rn.f32x2 %0, %1, %2, %3;"
@@ -1321,6 +1331,14 @@ __device__ __forceinline__ void finish_agent(const Params<T>& P, const int s, co
     to3<T>(P.POLD[s], xo);
     if (dist<T, D>(xn, xo) >= P.rebuild_thr) P.ctr->flag[p] = 1;
   }
+}
+
+// A CLVD step whose forces come from the cells alone: the list is stale, the
+// step's births or deaths will rebuild it, and every pair with a force lies
+// within the list radius.
+template <typename T>
+__device__ __forceinline__ bool clvd_walks_cells(const Params<T>& P) {
+  return P.ctr->events != 0 && !P.ctr->list_valid && P.force_in_list;
 }
 
 // Slot s of N; `list` is this thread's partner list (null: none); `live`
@@ -1729,7 +1747,11 @@ __device__ __forceinline__ void agent_de(const Params<T>& P, const int N, const 
 // the next launch.
 template <typename T, int D>
 __global__ void __launch_bounds__(kTile, sizeof(T) == 4 ? 4 : 3) k_agent_de(Params<T> P) {
+  pdl_wait();
   Counters* C = P.ctr;
+  if constexpr (D == 3) {
+    if (P.tiled && P.neighbors == CBM_NEIGH_CLVD && clvd_walks_cells(P)) return;
+  }
   const int N = (int)C->N[P.parity];
   if constexpr (!kPartnerLists<D>) {  // one thread per slot, grid over n_max
     const int slot = (int)blockIdx.x * kTile + (int)threadIdx.x;

@@ -1,0 +1,551 @@
+// cbm_tile.cuh — the 3D force walk by tiles of 32 agents.
+//
+// One warp owns 32 consecutive slots.  Slots are sorted by cell, so its agents
+// sit in one or a few cells of one row and share nearly all their candidates.
+// The filter (which candidates may lie within the cutoff) is a contraction:
+//     |xi - xj|^2 - R^2 = (|xi|^2 - R^2) + |xj|^2 - 2 xi . xj
+// over the coordinates relative to the tile, so 16 agents x 8 candidates are
+// one mma.m16n8k8 (half inputs, float accumulators), and the sign of an
+// accumulator is the decision: one funnel shift per pair collects it into a
+// word of 32 decisions (against about eleven instructions per pair when a
+// thread tests its own candidates).  The filter only has to keep every pair
+// that the evaluation's exact test keeps (see tile_row); the evaluation then
+// walks each agent's own words in candidate order and computes the terms
+// exactly as the reference does, so the sums are unchanged, bit for bit.
+#pragma once
+#include <cuda_fp16.h>
+
+#include "cbm_kernels.cuh"
+
+namespace cbm {
+
+// Decisions are kept as a ring of words of 32 candidates per agent: 27 cells
+// at 4 agents per unit volume (edge 3.3) are about 126 words.  The agents of
+// a tile find their partners in different parts of the walk (one near the
+// lower face of its cell mostly in the plane below), so each consumes its
+// words at its own pace, and the ring is refilled when the slowest has
+// consumed a third of it.  A ring of 48 words (6 KB a warp) and thirteen
+// warps an SM leave 124 KB of L1 to the partners' positions: measured on the
+// colony of 1e6 agents, 96 words and fifteen warps 2.28 ms (28 KB of L1), 80
+// and sixteen 2.14, 64 and sixteen 2.17 (60 KB), 48 and thirteen 2.05 (124
+// KB), 40 and fifteen 2.26, 40 and ten 2.31 (156 KB).
+constexpr int kTileWords = 48;
+constexpr int kTileRefill = 16;
+constexpr int kTileWarps = 13;    // one-warp blocks an SM
+constexpr int kTileCarveout = 58; // percent: 132 KB of shared memory
+static_assert(kTileWords % 4 == 0 && kTileRefill % 4 == 0, "the filter takes four words at a time");
+// bytes between the records of two words: 32 records of 16 bytes and a shift
+// of 8 banks, so that the eight rows of an ldmatrix (two records of each of
+// four words) fall into different banks
+constexpr int kTileWordStride = 32 * 16 + 32;
+// Largest |coordinate| relative to the tile that the half records hold with
+// the bounds of tile_row; farther agents and candidates are always kept.
+constexpr float kTileReach = 100.f;
+// cutoffs above this keep the per-thread walk (R^2 must stay far below the
+// largest half)
+constexpr double kTileMaxCutoff = 50.0;
+
+struct TileSmem {
+  unsigned word[(kTileWords + 1) * 32];  // decisions of word w, agent a; then an empty word
+  int base[kTileWords + 1];              // first slot of word w
+  unsigned short info[kTileWords];       // run (0..8) | number of candidates << 8
+  __align__(16) unsigned char rec[4 * kTileWordStride];  // records of four words
+};
+
+__device__ __forceinline__ unsigned half2_bits(float lo, float hi) {
+  const __half2 h = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const unsigned*>(&h);
+}
+
+__device__ __forceinline__ void ldmatrix4(unsigned* r, unsigned addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+
+// d = a b + (ca, ca, cb, cb): rows g and g + 8 of 16 agents against 8 candidates
+__device__ __forceinline__ void mma_16x8x8(float* d, unsigned a0, unsigned a1, unsigned b, float ca,
+                                           float cb) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
+      "{%7,%7,%8,%8};\n"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(b), "f"(ca), "f"(cb));
+}
+
+// A candidate's record, half (x, y | z, nh | nl, 0 | 0, 0) with nh + nl its
+// squared norm: the k dimension of the contraction.  A candidate out of reach
+// (or not a number) is kept whatever the agent, one beyond its run never.
+__device__ __forceinline__ uint4 tile_candidate(float x, float y, float z, bool valid, bool* far) {
+  const float hx = __half2float(__float2half_rn(x));
+  const float hy = __half2float(__float2half_rn(y));
+  const float hz = __half2float(__float2half_rn(z));
+  const float n = __fmaf_rn(hz, hz, __fmaf_rn(hy, hy, hx * hx));
+  const float nh = __half2float(__float2half_rn(n));
+  uint4 r = make_uint4(half2_bits(hx, hy), half2_bits(hz, nh), half2_bits(n - nh, 0.f), 0u);
+  // (a NaN fails the test of n, whatever fmaxf makes of it)
+  if (!(fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z)) <= kTileReach) || !(n < 60000.f)) {
+    r = make_uint4(0u, half2_bits(0.f, -60000.f), 0u, 0u);
+    *far = true;
+  }
+  if (!valid) r = make_uint4(0u, half2_bits(0.f, 65504.f), 0u, 0u);
+  return r;
+}
+
+// An agent's row, half (-2x, -2y | -2z, 1 | 1, 0 | 0, 0), and the start of its
+// accumulator, |x|^2 - R^2.  With u = 2^-11 (half rounding) and X the agent's
+// largest |coordinate|, a candidate inside the cutoff c has coordinates of at
+// most X + c, so each component of the difference of the rounded positions is
+// within E = u (2X + c) (plus float rounding) of the exact one, and the
+// rounded distance is below R = c + sqrt(3) E.  The contraction adds at most
+// six products that are exact in float: its roundings, and those of nh + nl
+// and of R, stay below 2^-18 (|x| + R)^2 for every pair closer than R; the
+// start is lowered by 2^-16 of it.  Agents out of reach keep every candidate
+// of their runs, lanes outside the tile's row none.
+__device__ __forceinline__ uint4 tile_row(float x, float y, float z, float c, bool member,
+                                          float* start) {
+  const float X = fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z));
+  const float hx = __half2float(__float2half_rn(x));
+  const float hy = __half2float(__float2half_rn(y));
+  const float hz = __half2float(__float2half_rn(z));
+  const float n = __fmaf_rn(hz, hz, __fmaf_rn(hy, hy, hx * hx));
+  const float R = c + 1.7320509f * (4.886e-4f * (2.f * X + c) + 3e-6f);
+  const float m = sqrtf(n) + R;
+  *start = n - R * R - 1.52587890625e-5f * (m * m);
+  uint4 r = make_uint4(half2_bits(-2.f * hx, -2.f * hy), half2_bits(-2.f * hz, 1.f),
+                       half2_bits(1.f, 0.f), 0u);
+  if (!(X <= kTileReach)) {
+    r = make_uint4(0u, half2_bits(0.f, 1.f), half2_bits(1.f, 0.f), 0u);
+    *start = -61000.f;
+  }
+  if (!member) {
+    r = make_uint4(0u, 0u, 0u, 0u);
+    *start = 1.f;
+  }
+  return r;
+}
+
+// The pair term in a form without branches: base and stiffness are selected,
+// and every pair beyond the cutoff, or the agent itself, adds a zero.  In
+// Float32 all of it is kept negated (-d^2, -d), which leaves no negations
+// between the packed operations.
+template <typename T>
+struct PairLine {
+  T nfar2, nreach, nrrep, krep, katt, rrep, abase;
+  bool mid;  // the stiffnesses are far from the ends of the exponent range
+};
+template <typename T>
+__device__ __forceinline__ PairLine<T> pair_line(const Params<T>& P) {
+  const bool rep = P.att_form == CBM_ATT_FROM_REP;
+  auto mid = [](T k) { return k == (T)0 || (fabs(k) > (T)1e-12 && fabs(k) < (T)1e12); };
+  // -(a (d - r)) and a (r - d) are the same number; so are -(a (c - d)) and
+  // (-a) (c - d).  A squared distance of cut2 is a distance >= the cutoff.
+  return PairLine<T>{-P.cut2, -(P.r_rep > P.r_att ? P.r_rep : P.r_att), -P.r_rep, P.k_rep,
+                     rep ? P.k_att : -P.k_att, P.r_rep, rep ? P.r_rep : P.r_att,
+                     mid(P.k_rep) && mid(P.k_att)};
+}
+
+// The terms of four partners at positions v, added to acc in order; an entry
+// that is the agent itself adds nothing.  `plain`: the positions are within
+// kTileReach of one another and L.mid holds.  Square root and quotient are
+// sqrt_mid and div_mid on pairs of values.
+template <typename T>
+__device__ __forceinline__ void pair_terms4(const PairCoef<T>& c, const PairLine<T>& L, bool plain,
+                                            const T* xi, const typename V4T<T>::type* v, int s,
+                                            const int* qq, T* acc) {
+  if constexpr (std::is_same<T, float>::value) {
+    const float2 ixy = make_float2(xi[0], xi[1]);
+    float2 exy[4], n2[2];
+    float ez[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      exy[u] = f2_sub(ixy, make_float2(v[u].x, v[u].y));
+      ez[u] = xi[2] - v[u].z;
+      const float2 q = f2_mul(exy[u], exy[u]);
+      const float n = (-q.x - q.y) - ez[u] * ez[u];
+      (u & 1 ? n2[u >> 1].y : n2[u >> 1].x) = qq[u] == s ? L.nfar2 : n;
+    }
+    // coincident agents take the general form
+    if (plain && fmaxf(fmaxf(n2[0].x, n2[0].y), fmaxf(n2[1].x, n2[1].y)) < -1e-12f) {
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        const float2 x = n2[p], half = make_float2(0.5f, 0.5f);
+        float2 y;
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(-x.x));
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(-x.y));
+        float2 g = f2_mul(x, y), h = f2_mul(half, y);
+        float2 r = f2_fma(g, h, half);
+        g = f2_fma(g, r, g);
+        h = f2_fma(h, r, h);
+        const float2 d = f2_fma(f2_fma(g, g, x), h, g);  // minus the distances
+        const bool r0 = d.x > L.nrrep, r1 = d.y > L.nrrep;
+        const float2 k = make_float2(r0 ? L.krep : L.katt, r1 ? L.krep : L.katt);
+        const float2 b = make_float2(r0 ? L.rrep : L.abase, r1 ? L.rrep : L.abase);
+        const float2 F = f2_mul(k, f2_add(b, d));
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(-d.x));
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(-d.y));
+        y = f2_fma(y, f2_fma(d, y, make_float2(1.f, 1.f)), y);
+        float2 q = f2_mul(F, y);
+        q = f2_fma(f2_fma(d, q, F), y, q);
+        const float c0 = d.x > L.nreach ? q.x : 0.f, c1 = d.y > L.nreach ? q.y : 0.f;
+        const float2 t0 = f2_mul(make_float2(c0, c0), exy[2 * p]);
+        const float2 t1 = f2_mul(make_float2(c1, c1), exy[2 * p + 1]);
+        // scalar sums: a packed product and a packed sum came out fused
+        acc[0] = (acc[0] + t0.x) + t1.x;
+        acc[1] = (acc[1] + t0.y) + t1.y;
+        acc[2] = (acc[2] + c0 * ez[2 * p]) + c1 * ez[2 * p + 1];
+      }
+      return;
+    }
+  }
+  if constexpr (std::is_same<T, double>::value) {
+    double e[4][3], n2[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      double xj[3];
+      to3<double>(v[u], xj);
+      const double d2 = pair_diff<double, 3>(xi, xj, e[u]);
+      n2[u] = qq[u] == s ? -L.nfar2 : d2;
+    }
+    if (plain && fmin(fmin(n2[0], n2[1]), fmin(n2[2], n2[3])) > 1e-12) {
+      double sc[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        double y;
+        const double d = sqrt_mid(n2[u], &y);
+        const bool rep = d < -L.nrrep;
+        const double F = (rep ? L.krep : L.katt) * ((rep ? L.rrep : L.abase) - d);
+        const double q = div_mid(F, d, y);
+        sc[u] = d < -L.nreach ? q : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) acc[k] = acc[k] + sc[u] * e[u][k];
+      return;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+    if (qq[u] != s) {
+      T xj[3], e[3];
+      to3<T>(v[u], xj);
+      const T d2 = pair_diff<T, 3>(xi, xj, e);
+      pair_term<T, 3>(c, e, d2, acc);
+    }
+}
+
+// The pair forces of the 32 slots from s0 on (lanes beyond N idle), summed
+// into acc in the reference's order.
+template <typename T>
+__device__ __forceinline__ void tile_forces(const Params<T>& P, TileSmem& S, const int N,
+                                            const int s0, const T* xi, T* acc) {
+  using V4 = typename V4T<T>::type;
+  const int lane = threadIdx.x & 31;
+  const bool in = s0 + lane < N;
+  const int s = in ? s0 + lane : N - 1;
+  const V4* const U = P.PA;
+  const PairCoef<T> coef = pair_coef<T>(P);
+  const int nx = P.n_cells_d[0], ny = P.n_cells_d[1], nz = P.n_cells_d[2];
+  const int cell = ld(P.cell_of_slot + s);
+  const int q0 = cell % nx, q1 = (cell / nx) % ny, q2 = cell / (nx * ny);
+  // the nine runs of the agent's 27 cells: rows (dy, dz), each the slots of
+  // up to three cells along x
+  const int xa = q0 > 0 ? q0 - 1 : 0, xb = q0 < nx - 1 ? q0 + 1 : nx - 1;
+  const int row0 = nx * (q1 - 1 + ny * (q2 - 1));
+  int lo[9], hi[9], cand = 0;
+#pragma unroll
+  for (int r = 0; r < 9; ++r) {
+    const int py = q1 + r % 3 - 1, pz = q2 + r / 3 - 1;
+    lo[r] = hi[r] = 0;
+    if (py >= 0 && py < ny && pz >= 0 && pz < nz) {
+      const int row = row0 + nx * (r % 3 + ny * (r / 3));
+      lo[r] = ld(P.cell_start + row + xa);
+      hi[r] = ld(P.cell_start + row + xb + 1);
+    }
+    cand += hi[r] - lo[r];
+  }
+  // agents of the same row of cells share their nine runs (up to their ends
+  // along x): the tile is processed row by row
+  const unsigned live = __ballot_sync(kFull, in);
+  const unsigned peers = __match_any_sync(kFull, in ? cell / nx : -1);
+  const unsigned leaders = __ballot_sync(kFull, in && (peers & ((1u << lane) - 1u)) == 0u);
+  const int n_rows = __popc(leaders);
+  const int cell0 = __shfl_sync(kFull, cell, 0);
+  const bool ranged = __any_sync(kFull, in && cell != cell0);
+  int u0 = 0, u1 = 0;  // lane r < 9: the run r of the current row of agents
+  auto unite = [&](unsigned gm) -> int {
+    const bool member = (gm >> lane) & 1u;
+    int words = 0;
+#pragma unroll
+    for (int r = 0; r < 9; ++r) {
+      const int a = __reduce_min_sync(kFull, member && hi[r] > lo[r] ? lo[r] : 0x7fffffff);
+      const int b = __reduce_max_sync(kFull, member ? hi[r] : 0);
+      const int len = b > a ? b - a : 0;
+      words += (len + 31) >> 5;
+      if (lane == r) {
+        u0 = len ? a : 0;
+        u1 = len ? b : 0;
+      }
+    }
+    return words;
+  };
+  // A word costs the warp about 75 instructions, a row of agents about 350,
+  // and a candidate tested by each lane about 14: sparse tiles, whose agents
+  // lie in many cells with a few candidates each, test their own.
+  const int most = __reduce_max_sync(kFull, in ? cand : 0);
+  bool by_tile = 14 * most > 350 * n_rows;
+  if (by_tile) {
+    int words = 0;
+    for (unsigned l = leaders; l; l &= l - 1u)
+      words += unite(__shfl_sync(kFull, peers, __ffs(l) - 1));
+    by_tile = 75 * words + 350 * n_rows < 14 * most;
+  }
+  const PairLine<T> line = pair_line(P);
+  if (!by_tile) {
+    if (!in) return;
+#pragma unroll
+    for (int r = 0; r < 9; ++r)
+      for (int q = lo[r]; q < hi[r]; q += 4) {  // beyond the run: the agent itself
+        int qq[4];
+        V4 v[4];
+        bool near = false, plain = line.mid;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) qq[u] = q + u < hi[r] ? q + u : s;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = U[qq[u]];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          T xj[3], e[3];
+          to3<T>(v[u], xj);
+          const T d2 = pair_diff<T, 3>(xi, xj, e);
+          near = near || (qq[u] != s && !(d2 >= coef.cut2));
+          plain = plain && d2 < (T)1e12;
+        }
+        if (near) pair_terms4<T>(coef, line, plain, xi, v, s, qq, acc);
+      }
+    return;
+  }
+
+  const float c = sqrtf((float)P.cut2) * 1.000002f;
+  const int g = lane >> 2, q4 = lane & 3;
+  const unsigned rec = (unsigned)__cvta_generic_to_shared(S.rec);
+  unsigned row_a[4];       // A fragments: agents 0-7, 8-15, 16-23, 24-31
+  float start[4];          // accumulator starts of agents g, g + 8, g + 16, g + 24
+  T org[3];
+  bool member = false;
+  unsigned rem = leaders;
+  int run = 9, k0 = 0, k1 = 0;   // next candidate and end of the run being queued
+  // words are counted from 0; word n sits at n modulo kTileWords.  made:
+  // words filtered; free_to: the ring has room below it; next: this lane's
+  // next word, at ring position `at`; bits: what is left of its current word.
+  int made = 0, ring = 0, free_to = kTileWords, next = 0, at = 0, base = 0;
+  unsigned bits = 0u;
+  bool far = false;  // a candidate or agent out of reach
+  for (;;) {
+    while (made < free_to && (run < 9 || rem)) {
+      if (run == 9) {  // the next row of agents
+        const int lead = __ffs(rem) - 1;
+        const unsigned gm = __shfl_sync(kFull, peers, lead);
+        rem &= rem - 1u;
+        member = (gm >> lane) & 1u;
+        if (n_rows > 1) unite(gm);
+        // coordinates relative to the middle of the row's cells
+        const int qa = __shfl_sync(kFull, q0, lead), qb = __shfl_sync(kFull, q0, 31 - __clz(gm));
+        org[0] = P.box_lo[0] + ((T)(qa + qb) * (T)0.5 - (T)0.5) * P.edge;
+        org[1] = P.box_lo[1] + ((T)__shfl_sync(kFull, q1, lead) - (T)0.5) * P.edge;
+        org[2] = P.box_lo[2] + ((T)__shfl_sync(kFull, q2, lead) - (T)0.5) * P.edge;
+        float st;
+        far = far || !(fabs(xi[0] - org[0]) + fabs(xi[1] - org[1]) + fabs(xi[2] - org[2]) <= (T)kTileReach);
+        const uint4 a = tile_row((float)(xi[0] - org[0]), (float)(xi[1] - org[1]),
+                                 (float)(xi[2] - org[2]), c, member, &st);
+        *reinterpret_cast<uint4*>(S.rec + lane * 16) = a;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) start[k] = __shfl_sync(kFull, st, g + 8 * k);
+        __syncwarp();
+        ldmatrix4(row_a, rec + lane * 16);
+        __syncwarp();
+        run = 0;
+        k0 = __shfl_sync(kFull, u0, 0);
+        k1 = __shfl_sync(kFull, u1, 0);
+        if (member) {  // the words before are other agents'
+          next = made;
+          at = ring;
+        }
+      }
+      // queue words of the row's runs, as many as there is room for
+      int n = 0, pos = ring;
+      while (run < 9 && made + n < free_to) {
+        const int left = (k1 - k0 + 31) >> 5, room = free_to - made - n;
+        const int take = left < room ? left : room;
+        for (int k = lane; k < take; k += 32) {
+          const int b = k0 + 32 * k;
+          int w = pos + k;
+          w = w >= kTileWords ? w - kTileWords : w;
+          S.base[w] = b;
+          S.info[w] = (unsigned short)(run | ((k1 - b < 32 ? k1 - b : 32) << 8));
+        }
+        n += take;
+        pos += take;
+        pos = pos >= kTileWords ? pos - kTileWords : pos;
+        k0 += 32 * take;
+        if (k0 >= k1) {
+          ++run;
+          k0 = __shfl_sync(kFull, u0, run);
+          k1 = __shfl_sync(kFull, u1, run);
+        }
+      }
+      for (; n & 3; ++n) {  // whole groups of four
+        S.base[pos] = 0;
+        S.info[pos] = 0;
+        ++pos;
+      }
+      __syncwarp();
+      // filter: four words (128 candidates) at a time; lane `lane` prepares
+      // candidate `lane` of each word, and the loads of the next four words
+      // are in flight while these are multiplied
+      V4 v[4];
+      auto fetch = [&](int w) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          v[j] = U[lane < (S.info[w + j] >> 8) ? S.base[w + j] + lane : s];
+      };
+      int w = ring, cur = -1, rlo = 0, rhi = 0;
+      if (n) fetch(w);
+      for (int k = 0; k < n; k += 4) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          T xj[3];
+          to3<T>(v[j], xj);
+          *reinterpret_cast<uint4*>(S.rec + j * kTileWordStride + lane * 16) =
+              tile_candidate((float)(xj[0] - org[0]), (float)(xj[1] - org[1]),
+                             (float)(xj[2] - org[2]), lane < (S.info[w + j] >> 8), &far);
+        }
+        __syncwarp();
+        const int wn = w + 4 == kTileWords ? 0 : w + 4;
+        if (k + 4 < n) fetch(wn);
+        // column n of multiplication t is candidate 2t + (n & 1) of word n / 2:
+        // thread (g, q4) then holds candidates 2t and 2t + 1 of word q4
+        const unsigned addr = rec + ((lane & 7) >> 1) * kTileWordStride + (lane & 1) * 16 +
+                              (lane >> 3) * 32;
+        unsigned m[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (int t4 = 0; t4 < 4; ++t4) {
+          unsigned b[4];
+          ldmatrix4(b, addr + t4 * 128);
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            float d[8];
+            mma_16x8x8(d, row_a[0], row_a[1], b[t], start[0], start[1]);
+            mma_16x8x8(d + 4, row_a[2], row_a[3], b[t], start[2], start[3]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              m[i] = __funnelshift_l(__float_as_uint(d[2 * i]), m[i], 1);
+              m[i] = __funnelshift_l(__float_as_uint(d[2 * i + 1]), m[i], 1);
+            }
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) S.word[(w + q4) * 32 + g + 8 * i] = m[i];
+        __syncwarp();
+        if (ranged && member) {  // keep the agent's own cells of the shared runs
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int r = S.info[w + j] & 255, b = S.base[w + j];
+            if (r != cur) {
+              cur = r;
+              const int row = row0 + nx * (r % 3 + ny * (r / 3));
+              rlo = ld(P.cell_start + row + xa);
+              rhi = ld(P.cell_start + row + xb + 1);
+            }
+            const int skip = rlo - b, keep = rhi - b;
+            unsigned own = 0xffffffffu;
+            if (skip > 0) own = skip < 32 ? own >> skip : 0u;
+            if (keep < 32) own &= keep > 0 ? ~(0xffffffffu >> keep) : 0u;
+            S.word[(w + j) * 32 + lane] &= own;
+          }
+        }
+        w = wn;
+      }
+      ring = w;
+      made += n;
+    }
+    const bool last = run == 9 && rem == 0u;
+
+    // evaluation: each lane walks its own words, four partners at a time (the
+    // positions of four are in flight together; their terms are added in
+    // order), until the slowest has freed kTileRefill words, or to the end.
+    // The next word is read one ahead of its use; position kTileWords is empty.
+    const bool plain = line.mid && !__any_sync(kFull, far);
+    const int goal = last ? made : free_to - kTileWords + kTileRefill;
+    unsigned nbits;
+    int nbase;
+    auto read = [&]() {
+      const int p = next < made ? at : kTileWords;
+      nbits = S.word[p * 32 + lane];
+      nbase = S.base[p];
+    };
+    read();
+    while (__any_sync(kFull, next < goal || (last && bits != 0u))) {
+      int qq[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool adv = bits == 0u;
+        bits = adv ? nbits : bits;
+        base = adv ? nbase : base;
+        const int step = adv && next < made ? 1 : 0;
+        next += step;
+        at += step;
+        at = at == kTileWords ? 0 : at;
+        read();
+        const int k = __clz(bits);
+        qq[u] = bits ? base + k : s;
+        bits &= ~(0x80000000u >> (k & 31));
+      }
+      V4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = U[qq[u]];
+      pair_terms4<T>(coef, line, plain, xi, v, s, qq, acc);
+    }
+    if (last) return;
+    free_to += kTileRefill;
+  }
+}
+
+// agentStepDE! over the cell walk in 3D: CellLinked, and CLVD in a step with
+// births or deaths (every other CLVD step is k_agent_de's).  One warp a
+// block, as many as are resident; tile t is block t's, further ones come from
+// a ticket counter that the last block to finish resets.
+template <typename T>
+__global__ void __launch_bounds__(32, kTileWarps) k_agent_de_tile(Params<T> P) {
+  __shared__ TileSmem S;
+  pdl_wait();
+  Counters* C = P.ctr;
+  if (P.neighbors == CBM_NEIGH_CLVD && !clvd_walks_cells(P)) return;
+  const int N = (int)C->N[P.parity];
+  const int n_tiles = (N + 31) >> 5;
+  const int lane = threadIdx.x & 31;
+  S.word[kTileWords * 32 + lane] = 0u;
+  S.base[kTileWords] = 0;
+  int tile = (int)blockIdx.x;
+  while (tile < n_tiles) {
+    const int s = tile * 32 + lane;
+    T xi[3], acc[3] = {(T)0, (T)0, (T)0};
+    to3<T>(P.PA[s < N ? s : N - 1], xi);
+    tile_forces<T>(P, S, N, tile * 32, xi, acc);
+    if (s < N) finish_agent<T, 3>(P, s, xi, acc);
+    __syncwarp();
+    int t = 0;
+    if (lane == 0) t = (int)atomicAdd(&C->de_ticket, 1u);
+    tile = (int)gridDim.x + __shfl_sync(kFull, t, 0);
+  }
+  if (lane == 0) {
+    __threadfence();
+    if (atomicAdd(&C->de_done, 1u) == gridDim.x - 1) {
+      C->de_ticket = 0u;
+      C->de_done = 0u;
+    }
+  }
+}
+
+}  // namespace cbm
