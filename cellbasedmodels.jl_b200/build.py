@@ -20,7 +20,7 @@ DEPS = SOURCES + [
     os.path.join(HERE, "csrc", "cbm_common.cuh"),
     os.path.join(HERE, "csrc", "cbm_grid.cuh"),
     os.path.join(HERE, "csrc", "cbm_small.cuh"),
-    os.path.join(HERE, "csrc", "cbm_stencil_tma.cuh"),
+    os.path.join(HERE, "csrc", "cbm_stencil_vec.cuh"),
     os.path.join(HERE, "csrc", "cbm_tile.cuh"),
     os.path.join(HERE, "..", "include", "cbm_b200.h"),
     os.path.join(HERE, "..", "include", "cbm_rng.h"),

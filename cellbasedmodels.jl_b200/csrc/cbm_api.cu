@@ -17,34 +17,34 @@
 #include "../../include/cbm_b200.h"
 #include "cbm_kernels.cuh"
 #include "cbm_small.cuh"
-#include "cbm_stencil_tma.cuh"
+#include "cbm_stencil_vec.cuh"
 #include "cbm_tile.cuh"
 #include <utility>
 
 using namespace cbm;
 
 // Steps of one chained step graph, replayed by cbm_step calls of at least
-// this many steps when the medium has a gradient: inside the chain each
-// step's update runs beside the next step's gradient.  Even, so that a chain
-// leaves the parity as it found it.
+// this many steps when there is a medium: inside the chain the field's
+// kernels and the agents' kernels run as two pipelines that wait for each
+// other only where they share a buffer.  Even, so that a chain leaves the
+// parity as it found it.
 constexpr int kChainSteps = 8;
 static_assert(kChainSteps % 2 == 0, "a chain must keep the parity");
-// Media of at most this many nodes are chained.  Their gradient is short
-// next to the update it overlaps (1024^2 nodes: about 12 us against about
-// 35); the gradient of a 256^3 field is an HBM-bound kernel of about 50 us,
-// and chaining it measured slower.
-constexpr long long kChainMaxNodes = 1ll << 22;
+
+// The exchange in agent order takes lists (k_medium_links, k_medium_apply)
+// when the field has at least this many nodes per (agent, stencil node), else
+// the gather over the field's patches (k_secrete_rows).
+constexpr unsigned long long kListNodes = 4;
 
 struct cbm_ctx {
   cbm_config cfg{};
   int device = 0;
   cudaStream_t stream = nullptr;
-  // with a medium: the force kernel's branch of a step, forked from and
-  // joined to `stream` by events (the kernel shares no buffer with the
-  // medium kernels it overlaps); with a gradient as well, the branch of the
-  // next step's gradient inside a chained step graph
-  cudaStream_t side = nullptr, side2 = nullptr;
-  cudaEvent_t fork_ev = nullptr, join_ev = nullptr, grad_fork_ev = nullptr, grad_ev = nullptr;
+  // with a medium: the agents' pipeline of a step, forked from and joined to
+  // `stream`, which keeps the field's, and the events between the two
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork_ev = nullptr, join_ev = nullptr, links_ev = nullptr, field_ev = nullptr,
+              de_ev = nullptr, update_ev = nullptr;
   size_t tsize = 4;
   std::string err;
   std::vector<void*> allocs;
@@ -86,10 +86,12 @@ struct cbm_ctx {
   // medium
   void* c[2] = {};
   void* grad[2][3] = {};
-  int* gather_box = nullptr;  // cell-box tables of the secretion gather (k_gather_box)
-  // 3D medium: tensor maps of c[0] and c[1] for the TMA-fed stencils
-  CUtensorMap tmap_c[2];
-  bool tma_medium = false;
+  int* gather_box = nullptr;  // cell-box tables of the exchange's gather (k_gather_box)
+  // exchange by lists: buckets' first entries, entries, Float64 weights
+  unsigned* link_head = nullptr;
+  unsigned link_buckets = 0;
+  uint4* link = nullptr;
+  void* link_w = nullptr;
   Counters* ctr = nullptr;
   Counters* h_ctr = nullptr;   // pinned staging of the counters an upload writes
   int* scratch_int = nullptr;  // n_max ints for inspection calls
@@ -285,6 +287,12 @@ Params<T> params(const cbm_ctx* c, int parity) {
   P.cell_count = c->cell_count;
   P.cell_start = c->cell_start;
   P.gather_box = c->gather_box;
+  P.link_head = c->link_head;
+  P.link_mask = c->link_buckets ? c->link_buckets - 1u : 0u;
+  P.link_shift = 35;
+  for (unsigned b = c->link_buckets; b > 1; b >>= 1) --P.link_shift;
+  P.link = c->link;
+  P.link_w = (T*)c->link_w;
   P.scan_state = c->scan_state;
   P.nbr_n = c->nbr_n;
   P.nbr_list = c->nbr_list;
@@ -367,16 +375,16 @@ Params<T> params(const cbm_ctx* c, int parity) {
 
 // agents add to the medium (secretion) or take from it (uptake)
 bool exchanges(const cbm_config& k) { return k.medium && (k.secretion != 0 || k.uptake != 0); }
-bool uses_gather(const cbm_config& k) {
+bool orders_exchange(const cbm_config& k) {
   return exchanges(k) && k.medium_sampling == CBM_MEDIUM_BILINEAR &&
          k.neighbors == CBM_NEIGH_CELL_LINKED;
 }
 bool rule_needed(const cbm_config& k) {
-  return k.walls == CBM_WALLS_REFLECT || (exchanges(k) && !uses_gather(k)) ||
+  return k.walls == CBM_WALLS_REFLECT || (exchanges(k) && !orders_exchange(k)) ||
          k.fate != CBM_FATE_NONE;
 }
 // the atomic rule path reads the committed field from a snapshot
-bool needs_snapshot(const cbm_config& k) { return k.uptake != 0 && exchanges(k) && !uses_gather(k); }
+bool needs_snapshot(const cbm_config& k) { return k.uptake != 0 && exchanges(k) && !orders_exchange(k); }
 
 double cutoff(const cbm_config& k) { return k.r_rep > k.r_att ? k.r_rep : k.r_att; }
 
@@ -405,12 +413,10 @@ dim3 stencil_grid(const cbm_ctx* c) {
   return dim3((unsigned)((nx + kStX - 1) / kStX), (unsigned)((ny + kStTileY - 1) / kStTileY));
 }
 
-// z planes per block of the 3D stencils: about twelve blocks for every SM
-// (two to three waves of the TMA-fed blocks, five or six of which are
-// resident; each block works through its planes one after another, so more
-// and shorter runs keep more planes in flight: measured 0.061 ms at four,
-// 0.051 ms at twelve for the 256^3 FTCS step), and runs of at least 8
-// planes (each run also reads the two planes that close it)
+// z planes per block of the tiled 3D stencils: about twelve blocks for every
+// SM (each block works through its planes one after another, so more and
+// shorter runs keep more planes in flight), and runs of at least 8 planes
+// (each run also reads the two planes that close it)
 int stencil_z_run(const cbm_ctx* c) {
   const dim3 g = stencil_grid(c);
   const long long xy = (long long)g.x * g.y;
@@ -422,59 +428,34 @@ int stencil_z_run(const cbm_ctx* c) {
   if (z_run < 8) z_run = 8;
   return (int)z_run;
 }
+// The vector stencils: rows of whole 16-byte vectors.
+bool vec_medium(const cbm_ctx* c) {
+  return ((size_t)c->cfg.n_medium[0] * c->tsize) % 16 == 0;
+}
+int vec_blocks(const cbm_ctx* c) {
+  return grid_blocks((long long)c->cfg.n_medium[0] * (long long)c->tsize / 16 * c->cfg.n_medium[1]);
+}
+// planes a run: about sixteen blocks of 256 for every SM (two to three waves;
+// eight an SM measured 36 and 61 us for the two at 256^3 Float32, sixteen 34
+// and 49), and runs of at least 4 planes
+int vec_z_run(const cbm_ctx* c) {
+  const int nz = c->cfg.n_medium[2] > 0 ? c->cfg.n_medium[2] : 1;
+  const int xy = vec_blocks(c);
+  const long long want = 16LL * (c->n_sm > 0 ? c->n_sm : 148);
+  const long long runs = (want + xy - 1) / xy;
+  const int z_run = (int)((nz + runs - 1) / runs);
+  return z_run < 4 ? 4 : z_run;
+}
+dim3 vec_grid(const cbm_ctx* c) {
+  const int nz = c->cfg.n_medium[2] > 0 ? c->cfg.n_medium[2] : 1, zr = vec_z_run(c);
+  return dim3((unsigned)vec_blocks(c), (unsigned)((nz + zr - 1) / zr));
+}
 dim3 stencil_grid_3d(const cbm_ctx* c) {
   dim3 g = stencil_grid(c);
   const int nz = c->cfg.n_medium[2] > 0 ? c->cfg.n_medium[2] : 1;
   const int zr = stencil_z_run(c);
   g.z = (unsigned)((nz + zr - 1) / zr);
   return g;
-}
-
-// Tensor maps of the two medium buffers for the TMA-fed 3D stencils: the
-// field as an (nx, ny, nz) array of reals, boxes of one plane of a column
-// tile (TmaPlane), zeros outside.  Needs rows of a multiple of 16 bytes (the
-// strides of a tensor map); other shapes keep the register-pipelined
-// stencils.  cuTensorMapEncodeTiled is reached through the runtime's driver
-// entry point, so the library does not link the driver library itself.
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled_fn() {
-  static EncodeTiledFn fn = []() -> EncodeTiledFn {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q{};
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) !=
-            cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      return nullptr;
-    return reinterpret_cast<EncodeTiledFn>(f);
-  }();
-  return fn;
-}
-
-template <typename T>
-bool encode_medium_maps(cbm_ctx* c) {
-  using G = TmaPlane<T>;
-  const cbm_config& k = c->cfg;
-  if (!k.medium || k.dims != 3) return false;
-  const unsigned long long nx = k.n_medium[0], ny = k.n_medium[1], nz = k.n_medium[2];
-  if ((nx * sizeof(T)) % 16 != 0) return false;
-  EncodeTiledFn enc = encode_tiled_fn();
-  if (!enc) return false;
-  const cuuint64_t dim[3] = {nx, ny, nz};
-  const cuuint64_t stride[2] = {nx * sizeof(T), nx * ny * sizeof(T)};
-  const cuuint32_t box[3] = {(cuuint32_t)G::kBX, (cuuint32_t)G::kBY, 1};
-  const cuuint32_t estride[3] = {1, 1, 1};
-  for (int q = 0; q < 2; ++q)
-    if (enc(&c->tmap_c[q],
-            sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3,
-            c->c[q], dim, stride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return false;
-  return true;
 }
 
 // ---- stage launches (enqueue only) -----------------------------------------
@@ -485,9 +466,8 @@ void enqueue_medium_rule(cbm_ctx* c, const Params<T>& P) {
     if (D == 2)
       k_medium_grad_2d<T><<<stencil_grid(c), dim3(kStX, kStY), 0, c->stream>>>(P);
     else if (D == 3)
-      if (c->tma_medium)
-        k_medium_grad_3d_tma<T><<<stencil_grid_3d(c), dim3(kStX, kStY), TmaPlane<T>::kSmem,
-                                  c->stream>>>(P, c->tmap_c[P.parity], stencil_z_run(c));
+      if (vec_medium(c))
+        k_medium_grad_3d_vec<T><<<vec_grid(c), kTile, 0, c->stream>>>(P, vec_z_run(c));
       else
         k_medium_grad_3d<T><<<stencil_grid_3d(c), dim3(kStX, kStY), 0, c->stream>>>(P, stencil_z_run(c));
     else
@@ -496,21 +476,34 @@ void enqueue_medium_rule(cbm_ctx* c, const Params<T>& P) {
 }
 
 template <typename T, int D>
-void enqueue_agent_rule(cbm_ctx* c, const Params<T>& P, bool pdl_gather = false) {
+void enqueue_links(cbm_ctx* c, const Params<T>& P) {
+  cudaMemsetAsync(c->link_head, 0xff, (size_t)c->link_buckets * 4, c->stream);
+  PROF("k_medium_links");
+  k_medium_links<T, D><<<grid_blocks(c->cfg.n_max << D), kTile, 0, c->stream>>>(P);
+}
+template <typename T, int D>
+void enqueue_apply(cbm_ctx* c, const Params<T>& P) {
+  PROF("k_medium_apply");
+  k_medium_apply<T, D><<<grid_blocks(c->cfg.n_max << D), kTile, 0, c->stream>>>(P);
+}
+template <typename T, int D>
+void enqueue_gather(cbm_ctx* c, const Params<T>& P) {
+  PROF("k_secrete_rows");
+  const int nm[3] = {c->cfg.n_medium[0], D > 1 ? c->cfg.n_medium[1] : 1,
+                     D > 2 ? c->cfg.n_medium[2] : 1};
+  const int py = (nm[1] + GatherPatch<D>::kY - 1) / GatherPatch<D>::kY;
+  constexpr int W = GatherPatch<D>::kWarps;
+  const dim3 grid((unsigned)((nm[0] + 31) / 32), (unsigned)((py + W - 1) / W),
+                  (unsigned)((nm[2] + GatherPatch<D>::kZ - 1) / GatherPatch<D>::kZ));
+  k_secrete_rows<T, D><<<grid, W * 32, 0, c->stream>>>(P);
+}
+// walls, births and deaths, and the exchange that atomics add
+template <typename T, int D>
+void enqueue_rule(cbm_ctx* c, const Params<T>& P) {
   const cbm_config& k = c->cfg;
   if (needs_snapshot(k)) {
     PROF("k_medium_snapshot");
     k_medium_snapshot<T><<<grid_blocks(c->n_nodes), kTile, 0, c->stream>>>(P);
-  }
-  if (uses_gather(k)) {
-    PROF("k_secrete_rows");
-    const int nm[3] = {c->cfg.n_medium[0], D > 1 ? c->cfg.n_medium[1] : 1,
-                       D > 2 ? c->cfg.n_medium[2] : 1};
-    const int py = (nm[1] + GatherPatch<D>::kY - 1) / GatherPatch<D>::kY;
-    constexpr int W = GatherPatch<D>::kWarps;
-    const dim3 grid((unsigned)((nm[0] + 31) / 32), (unsigned)((py + W - 1) / W),
-                    (unsigned)((nm[2] + GatherPatch<D>::kZ - 1) / GatherPatch<D>::kZ));
-    launch_pdl(c, pdl_gather, k_secrete_rows<T, D>, grid, dim3(W * 32), 0, P);
   }
   if (!rule_needed(k)) return;
   if (k.fate != CBM_FATE_NONE) {
@@ -520,6 +513,16 @@ void enqueue_agent_rule(cbm_ctx* c, const Params<T>& P, bool pdl_gather = false)
     PROF("k_agent_rule");
     k_agent_rule<T, D><<<c->n_blocks, kTile, 0, c->stream>>>(P);
   }
+}
+template <typename T, int D>
+void enqueue_agent_rule(cbm_ctx* c, const Params<T>& P) {
+  if (c->link_buckets) {
+    enqueue_links<T, D>(c, P);
+    enqueue_apply<T, D>(c, P);
+  } else if (orders_exchange(c->cfg)) {
+    enqueue_gather<T, D>(c, P);
+  }
+  enqueue_rule<T, D>(c, P);
 }
 
 template <typename T, int D>
@@ -577,20 +580,18 @@ void enqueue_agent_de(cbm_ctx* c, const Params<T>& P) {
 }
 
 template <typename T, int D>
-void enqueue_medium_de(cbm_ctx* c, const Params<T>& P, bool pdl = false) {
+void enqueue_medium_de(cbm_ctx* c, const Params<T>& P) {
   if (c->cfg.medium) {
     PROF("k_medium_de");
     if (D == 2)
-      launch_pdl(c, pdl, k_medium_de_2d<T>, stencil_grid(c), dim3(kStX, kStY), 0, P);
+      k_medium_de_2d<T><<<stencil_grid(c), dim3(kStX, kStY), 0, c->stream>>>(P);
     else if (D == 3)
-      if (c->tma_medium)
-        launch_pdl(c, pdl, k_medium_de_3d_tma<T>, stencil_grid_3d(c), dim3(kStX, kStY),
-                   (size_t)TmaPlane<T>::kSmem, P, c->tmap_c[P.parity], stencil_z_run(c));
+      if (vec_medium(c))
+        k_medium_de_3d_vec<T><<<vec_grid(c), kTile, 0, c->stream>>>(P, vec_z_run(c));
       else
-        launch_pdl(c, pdl, k_medium_de_3d<T>, stencil_grid_3d(c), dim3(kStX, kStY), 0, P,
-                   stencil_z_run(c));
+        k_medium_de_3d<T><<<stencil_grid_3d(c), dim3(kStX, kStY), 0, c->stream>>>(P, stencil_z_run(c));
     else
-      launch_pdl(c, pdl, k_medium_de<T, D>, dim3(grid_blocks(c->n_nodes)), dim3(kTile), 0, P);
+      k_medium_de<T, D><<<grid_blocks(c->n_nodes), kTile, 0, c->stream>>>(P);
   }
 }
 
@@ -641,7 +642,7 @@ int kernels_per_step(const cbm_ctx* c) {
   int n = 0;
   if (k.medium && k.chemotaxis != 0) n += 1;
   if (needs_snapshot(k)) n += 1;
-  if (uses_gather(k)) n += 1;
+  if (orders_exchange(k)) n += c->link_buckets ? 2 : 1;  // the lists and their sums, or the gather
   if (rule_needed(k)) n += 1;           // rule (with births and deaths when fate is on)
   if (k.fate != CBM_FATE_NONE) n += 1;  // compaction
   n += 1;                               // agent DE
@@ -654,55 +655,77 @@ int kernels_per_step(const cbm_ctx* c) {
   return n;
 }
 
+// One step from parity `parity`; `first` and `last` of the steps enqueued
+// together.  With a medium they form two pipelines.  The field's, on `stream`:
+// gradient G, exchange A, FTCS F; the agents', on `side`: lists L of the
+// exchange, rule, force kernel D, update and neighbors U.  They wait for each
+// other where they share a buffer:
+//   A by lists needs L, and the next L (which writes the lists again) needs A;
+//   A by the gather, or as a rule that adds with atomics, reads the agents: it
+//   needs the U before it and the U after needs it; the rule is also needed by
+//   D, which reads the reflected positions;
+//   D reads the gradient of the step before, the next G writes that buffer.
+// U and F, which share nothing, overlap, and in a chain the two pipelines run
+// ahead of each other.  Per-kernel timing keeps the series order.  A failed
+// event call is seen like a failed launch (by the capture, or by
+// cudaGetLastError after an eager step).
 template <typename T, int D>
-void enqueue_full_step(cbm_ctx* c, int parity, bool grad_ahead = false, bool next_grad = false) {
+void enqueue_full_step(cbm_ctx* c, int parity, bool first = true, bool last = true) {
   Params<T> P = params<T>(c, parity);
-  // The force kernel reads the committed positions and gradient and writes
-  // the next state; the medium kernels read and write only the field and
-  // its gradient.  With a medium the two run as parallel branches: the
-  // force kernel on `side`, forked after the last kernel it depends on (the
-  // agents' rule when there is one, else at the start of the step) and
-  // joined before the update.  Per-kernel timing keeps them in series.  A
-  // failed event call is seen like a failed launch (by the capture, or by
-  // cudaGetLastError after an eager step).
-  const bool fork = c->side && !c->prof;
-  const bool early = fork && !rule_needed(c->cfg);
-  auto agent_de = [&] {
-    cudaEventRecord(c->fork_ev, c->stream);
-    cudaStreamWaitEvent(c->side, c->fork_ev, 0);
-    cudaStream_t main = c->stream;
-    c->stream = c->side;
+  const cbm_config& k = c->cfg;
+  if (!c->side || c->prof) {
+    enqueue_medium_rule<T, D>(c, P);
+    enqueue_agent_rule<T, D>(c, P);
     enqueue_agent_de<T, D>(c, P);
-    c->stream = main;
-    cudaEventRecord(c->join_ev, c->side);
-  };
-  if (early) agent_de();
-  // the gradient reads only the committed c: it may precede the secretion,
-  // and in a chained graph the previous step enqueued it beside its update
-  if (grad_ahead) cudaStreamWaitEvent(c->stream, c->grad_ev, 0);
-  else enqueue_medium_rule<T, D>(c, P);
-  // programmatic launches where the kernel before is one on this stream:
-  // the secretion after the gradient, the FTCS after the secretion
-  const bool grad_before = !grad_ahead && c->cfg.medium && c->cfg.chemotaxis != 0;
-  enqueue_agent_rule<T, D>(c, P, grad_before && !needs_snapshot(c->cfg));
-  if (!fork) enqueue_agent_de<T, D>(c, P);
-  else if (!early) agent_de();
-  enqueue_medium_de<T, D>(c, P, early && uses_gather(c->cfg) && !rule_needed(c->cfg));
-  if (fork) cudaStreamWaitEvent(c->stream, c->join_ev, 0);
-  if (next_grad) {
-    // The next step's gradient reads the field just written and writes the
-    // gradient buffer this step's force kernel has read (joined above); the
-    // update touches neither, so the two run side by side.
-    cudaEventRecord(c->grad_fork_ev, c->stream);
-    cudaStreamWaitEvent(c->side2, c->grad_fork_ev, 0);
-    cudaStream_t main = c->stream;
-    c->stream = c->side2;
-    enqueue_medium_rule<T, D>(c, params<T>(c, parity ^ 1));
-    c->stream = main;
-    cudaEventRecord(c->grad_ev, c->side2);
+    enqueue_medium_de<T, D>(c, P);
+    enqueue_update<T, D>(c, P);
+    enqueue_neighbors<T, D>(c, params<T>(c, parity ^ 1));
+    return;
   }
+  cudaStream_t field = c->stream, agents = c->side;
+  const bool lists = c->link_buckets != 0;
+  const bool gather = orders_exchange(k) && !lists;
+  const bool atomics = exchanges(k) && !orders_exchange(k);
+  const bool grad = k.chemotaxis != 0;
+  if (first) {
+    cudaEventRecord(c->fork_ev, field);
+    cudaStreamWaitEvent(agents, c->fork_ev, 0);
+  }
+  c->stream = agents;
+  // the last step's A (the lists) and G (the gradient D reads)
+  if (!first && (lists || grad)) cudaStreamWaitEvent(agents, c->field_ev, 0);
+  if (lists) {
+    enqueue_links<T, D>(c, P);
+    cudaEventRecord(c->links_ev, agents);
+  }
+  c->stream = field;
+  if (grad) {
+    if (!first) cudaStreamWaitEvent(field, c->de_ev, 0);
+    enqueue_medium_rule<T, D>(c, P);
+  }
+  if (lists) {
+    cudaStreamWaitEvent(field, c->links_ev, 0);
+    enqueue_apply<T, D>(c, P);
+  }
+  if ((gather || atomics) && !first) cudaStreamWaitEvent(field, c->update_ev, 0);
+  if (gather) enqueue_gather<T, D>(c, P);
+  if (atomics) enqueue_rule<T, D>(c, P);
+  cudaEventRecord(c->field_ev, field);
+  enqueue_medium_de<T, D>(c, P);
+  c->stream = agents;
+  if (atomics) cudaStreamWaitEvent(agents, c->field_ev, 0);
+  if (!atomics) enqueue_rule<T, D>(c, P);
+  enqueue_agent_de<T, D>(c, P);
+  cudaEventRecord(c->de_ev, agents);
+  if (gather) cudaStreamWaitEvent(agents, c->field_ev, 0);
   enqueue_update<T, D>(c, P);
   enqueue_neighbors<T, D>(c, params<T>(c, parity ^ 1));
+  cudaEventRecord(c->update_ev, agents);
+  c->stream = field;
+  if (last) {
+    cudaEventRecord(c->join_ev, agents);
+    cudaStreamWaitEvent(field, c->join_ev, 0);
+  }
 }
 
 // dispatch on (precision, dims)
@@ -751,13 +774,12 @@ template <typename T, int D>
 struct FullStep {
   static void run(cbm_ctx* c, int parity) { enqueue_full_step<T, D>(c, parity); }
 };
-// kChainSteps steps from parity p; each step after the first takes the
-// gradient its predecessor enqueued beside its update
+// kChainSteps steps from parity p
 template <typename T, int D>
 struct ChainSteps {
   static void run(cbm_ctx* c, int parity) {
     for (int i = 0; i < kChainSteps; ++i)
-      enqueue_full_step<T, D>(c, parity ^ (i & 1), i > 0, i + 1 < kChainSteps);
+      enqueue_full_step<T, D>(c, parity ^ (i & 1), i == 0, i + 1 == kChainSteps);
   }
 };
 template <typename T, int D>
@@ -876,11 +898,12 @@ void free_all(cbm_ctx* c) {
   c->h_ctr = nullptr;
   c->allocs.clear();
   if (c->side) cudaStreamDestroy(c->side);
-  if (c->side2) cudaStreamDestroy(c->side2);
-  for (cudaEvent_t e : {c->fork_ev, c->join_ev, c->grad_fork_ev, c->grad_ev})
-    if (e) cudaEventDestroy(e);
-  c->side = c->side2 = nullptr;
-  c->fork_ev = c->join_ev = c->grad_fork_ev = c->grad_ev = nullptr;
+  c->side = nullptr;
+  for (cudaEvent_t* e :
+       {&c->fork_ev, &c->join_ev, &c->links_ev, &c->field_ev, &c->de_ev, &c->update_ev}) {
+    if (*e) cudaEventDestroy(*e);
+    *e = nullptr;
+  }
   if (c->stream) cudaStreamDestroy(c->stream);
   c->stream = nullptr;
 }
@@ -983,33 +1006,20 @@ int cbm_create(cbm_ctx** out, const cbm_config* cfg) {
   c->tsize = k.precision == CBM_F64 ? 8 : 4;
   cudaGetDevice(&c->device);
   cudaDeviceGetAttribute(&c->n_sm, cudaDevAttrMultiProcessorCount, c->device);
-  // Chained step graphs (a medium with a gradient, of at most
-  // kChainMaxNodes nodes): the library's stream takes the greatest priority
-  // and the branches keep the least, so that the update and the medium
-  // chain go first and the force kernel and the next gradient fill the SMs
-  // they leave (with equal priorities the chained 1024^2 chemotaxis step
-  // measured 9-13 % slower).
-  long long med_nodes = 1;
-  for (int d = 0; d < k.dims && k.medium && med_nodes <= kChainMaxNodes; ++d)
-    med_nodes *= k.n_medium[d] > 0 ? k.n_medium[d] : 1;  // stops past the bound: no overflow
-  const bool chained = k.medium && k.chemotaxis != 0 && med_nodes <= kChainMaxNodes;
-  int prio_least = 0, prio_greatest = 0;
-  cudaError_t se = cudaDeviceGetStreamPriorityRange(&prio_least, &prio_greatest);
-  if (se == cudaSuccess)
-    se = chained ? cudaStreamCreateWithPriority(&c->stream, cudaStreamNonBlocking, prio_greatest)
-                 : cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
+  cudaError_t se = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (se != cudaSuccess) {
     int rc = fail(nullptr, CBM_ERR_CUDA, "cudaStreamCreate failed (is a CUDA device present?)");
     delete c;
     return rc;
   }
-  if ((k.medium && (cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess ||
-                    cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
-                    cudaEventCreateWithFlags(&c->join_ev, cudaEventDisableTiming) != cudaSuccess)) ||
-      (chained && (cudaStreamCreateWithFlags(&c->side2, cudaStreamNonBlocking) != cudaSuccess ||
-                   cudaEventCreateWithFlags(&c->grad_fork_ev, cudaEventDisableTiming) != cudaSuccess ||
-                   cudaEventCreateWithFlags(&c->grad_ev, cudaEventDisableTiming) != cudaSuccess))) {
-    int rc = fail(nullptr, CBM_ERR_CUDA, "creating the branch streams of the step graph failed");
+  if (k.medium) {
+    se = cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking);
+    for (cudaEvent_t* e :
+         {&c->fork_ev, &c->join_ev, &c->links_ev, &c->field_ev, &c->de_ev, &c->update_ev})
+      if (se == cudaSuccess) se = cudaEventCreateWithFlags(e, cudaEventDisableTiming);
+  }
+  if (se != cudaSuccess) {
+    int rc = fail(nullptr, CBM_ERR_CUDA, "creating the branch of the step graph failed");
     free_all(c);
     delete c;
     return rc;
@@ -1121,9 +1131,20 @@ int cbm_create(cbm_ctx** out, const cbm_config* cfg) {
       c->c[q] = dalloc(c, (size_t)c->n_nodes * S, &ok);
       for (int d = 0; d < 3; ++d) c->grad[q][d] = dalloc(c, (size_t)c->n_nodes * S, &ok);
     }
-    size_t nb = 0;
-    for (int d = 0; d < k.dims; ++d) nb += 2 * (size_t)k.n_medium[d];
-    c->gather_box = (int*)dalloc(c, nb * 4, &ok);
+    if (orders_exchange(k)) {
+      size_t nb = 0;
+      for (int d = 0; d < k.dims; ++d) nb += 2 * (size_t)k.n_medium[d];
+      c->gather_box = (int*)dalloc(c, nb * 4, &ok);
+    }
+    // an entry per agent and stencil node
+    const unsigned long long ne = (unsigned long long)n << k.dims;
+    if (orders_exchange(k) && ne * kListNodes <= (unsigned long long)c->n_nodes) {
+      c->link_buckets = 1024;
+      while (c->link_buckets < ne) c->link_buckets *= 2;
+      c->link_head = (unsigned*)dalloc(c, (size_t)c->link_buckets * 4, &ok);
+      c->link = (uint4*)dalloc(c, ne * sizeof(uint4), &ok);
+      if (S == 8) c->link_w = dalloc(c, ne * S, &ok);
+    }
   }
   c->ctr = (Counters*)dalloc(c, sizeof(Counters), &ok);
   if (ok && cudaMallocHost((void**)&c->h_ctr, sizeof(Counters)) != cudaSuccess) {
@@ -1136,8 +1157,7 @@ int cbm_create(cbm_ctx** out, const cbm_config* cfg) {
     delete c;
     return rc;
   }
-  c->tma_medium = c->tsize == 8 ? encode_medium_maps<double>(c) : encode_medium_maps<float>(c);
-  if (k.medium) {
+  if (c->gather_box) {
     int nmax = 1;
     for (int d = 0; d < k.dims; ++d) nmax = k.n_medium[d] > nmax ? (int)k.n_medium[d] : nmax;
     const unsigned blocks = (unsigned)((nmax + 255) / 256);
@@ -1215,11 +1235,17 @@ int cbm_upload(cbm_ctx* c, const cbm_state_view* h) {
   if (k.medium) {
     const size_t nb = (size_t)c->n_nodes * S;
     for (int q = 0; q < 2; ++q) {
-      if (h->medium_c) CUDA_TRY(c, cudaMemcpyAsync(c->c[q], h->medium_c, nb, cudaMemcpyHostToDevice, st));
+      // over the bus once; the second copy is the device's own
+      if (h->medium_c)
+        CUDA_TRY(c, q == 0 ? cudaMemcpyAsync(c->c[0], h->medium_c, nb, cudaMemcpyHostToDevice, st)
+                           : cudaMemcpyAsync(c->c[1], c->c[0], nb, cudaMemcpyDeviceToDevice, st));
       else CUDA_TRY(c, cudaMemsetAsync(c->c[q], 0, nb, st));
       for (int d = 0; d < 3; ++d) {
         if (d < k.dims && h->medium_grad[d])
-          CUDA_TRY(c, cudaMemcpyAsync(c->grad[q][d], h->medium_grad[d], nb, cudaMemcpyHostToDevice, st));
+          CUDA_TRY(c, q == 0 ? cudaMemcpyAsync(c->grad[0][d], h->medium_grad[d], nb,
+                                               cudaMemcpyHostToDevice, st)
+                             : cudaMemcpyAsync(c->grad[1][d], c->grad[0][d], nb,
+                                               cudaMemcpyDeviceToDevice, st));
         else CUDA_TRY(c, cudaMemsetAsync(c->grad[q][d], 0, nb, st));
       }
     }
@@ -1447,15 +1473,14 @@ int cbm_step(cbm_ctx* c, int32_t nsteps, int32_t flags) {
   }
   for (int s = 0; s < nsteps; ++s) {
     const int p = c->parity;
-    if (use_graph && !c->graph_timing && c->side2 && nsteps - s >= kChainSteps) {
+    if (use_graph && !c->graph_timing && c->side && nsteps - s >= kChainSteps) {
       if (!c->chain[p]) {
         cudaGraph_t g = nullptr;
         CUDA_TRY(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
         dispatch<ChainSteps>(c, p);
         cudaError_t e = cudaStreamEndCapture(c->stream, &g);
         if (e != cudaSuccess) return fail(c, CBM_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
-        // the nodes keep the priorities of the streams they were captured on
-        e = cudaGraphInstantiate(&c->chain[p], g, cudaGraphInstantiateFlagUseNodePriority);
+        e = cudaGraphInstantiate(&c->chain[p], g, 0);
         cudaGraphDestroy(g);
         if (e != cudaSuccess) return fail(c, CBM_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(e));
       }
