@@ -595,27 +595,40 @@ void enqueue_medium_de(cbm_ctx* c, const Params<T>& P) {
   }
 }
 
-// update!: compaction, commit, then B -> A (copy, or re-sort = grid rebuild)
+// In a step whose agents are neither born nor die and whose grid is rebuilt
+// every time, the force kernel files each agent in its new cell: the re-sort
+// then begins with the scan, which commits the counters.
+bool hist_in_de(const cbm_config& k) {
+  static_assert(kHistInDE<2> && !kHistInDE<3>, "as below");
+  return k.dims < 3 && k.neighbors == CBM_NEIGH_CELL_LINKED && k.fate == CBM_FATE_NONE &&
+         (k.integrator == CBM_INT_EULER || k.integrator == CBM_INT_EM);
+}
+
+// update!: compaction, then B -> A (copy, or re-sort = grid rebuild) with the
+// commit of the counters.  The kernels follow one another on the stream;
+// `after_kernel`: so does the first of them.
 template <typename T, int D>
-void enqueue_update(cbm_ctx* c, const Params<T>& P) {
+void enqueue_update(cbm_ctx* c, const Params<T>& P, bool after_kernel = false) {
   if (c->cfg.fate != CBM_FATE_NONE) {
     PROF("k_compact");
     k_compact<T, D><<<c->n_sm, kCompactThreads, 0, c->stream>>>(P);
+    after_kernel = true;
   }
-  {
-    PROF("k_commit");
-    k_commit<T><<<1, 1, 0, c->stream>>>(P);
-  }
-  // the four sort kernels follow one another on the stream
-  {
+  ScanArgs A{c->cell_count, c->cell_start, c->scan_state, c->n_cells, c->n_scan_tiles, c->ctr,
+             resort_flag(c)};
+  if (P.hist_in_de) {
+    A.due = nullptr;
+    A.commit = 1;
+    A.parity = P.parity;
+    A.dt = P.dt_time;
+  } else {
     PROF("k_sort_hist");
-    launch_pdl(c, true, k_sort_hist<T, D>, dim3(c->n_blocks), dim3(kTile), 0, P);
+    launch_pdl(c, after_kernel, k_sort_hist<T, D>, dim3(c->n_blocks), dim3(kTile), 0, P, 1);
+    after_kernel = true;
   }
   {
     PROF("k_scan_cells");
-    ScanArgs A{c->cell_count, c->cell_start, c->scan_state, c->n_cells, c->n_scan_tiles, c->ctr,
-               resort_flag(c)};
-    launch_pdl(c, true, k_scan_cells, dim3(c->n_scan_tiles), dim3(kTile), 0, A);
+    launch_pdl(c, after_kernel, k_scan_cells, dim3(c->n_scan_tiles), dim3(kTile), 0, A);
   }
   {
     PROF("k_sort_scatter");
@@ -650,7 +663,7 @@ int kernels_per_step(const cbm_ctx* c) {
   if (c->pos32) n += 1;                 // its Float32 positions (Float64 3D walks)
   if (c->pos_rows) n += 1;              // its position rows (Float32 3D walks)
   if (k.medium) n += 1;
-  n += 5;                               // commit, sort hist, scan, scatter, place
+  n += hist_in_de(k) ? 3 : 4;           // sort hist, scan, scatter, place
   if (k.neighbors == CBM_NEIGH_VERLET_DISPLACEMENT) n += 1;
   return n;
 }
@@ -673,12 +686,13 @@ template <typename T, int D>
 void enqueue_full_step(cbm_ctx* c, int parity, bool first = true, bool last = true) {
   Params<T> P = params<T>(c, parity);
   const cbm_config& k = c->cfg;
+  P.hist_in_de = hist_in_de(k) ? 1 : 0;
   if (!c->side || c->prof) {
     enqueue_medium_rule<T, D>(c, P);
     enqueue_agent_rule<T, D>(c, P);
     enqueue_agent_de<T, D>(c, P);
     enqueue_medium_de<T, D>(c, P);
-    enqueue_update<T, D>(c, P);
+    enqueue_update<T, D>(c, P, true);
     enqueue_neighbors<T, D>(c, params<T>(c, parity ^ 1));
     return;
   }
@@ -846,7 +860,7 @@ template <typename T, int D>
 struct FirstSort {  // the re-sort half of update!, for loadToPlatform!
   static void run(cbm_ctx* c) {
     Params<T> P = params<T>(c, c->parity);
-    k_sort_hist<T, D><<<c->n_blocks, kTile, 0, c->stream>>>(P);
+    k_sort_hist<T, D><<<c->n_blocks, kTile, 0, c->stream>>>(P, 0);
     ScanArgs A{c->cell_count, c->cell_start, c->scan_state, c->n_cells, c->n_scan_tiles, c->ctr,
                resort_flag(c)};
     k_scan_cells<<<c->n_scan_tiles, kTile, 0, c->stream>>>(A);

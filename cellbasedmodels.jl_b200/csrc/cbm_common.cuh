@@ -84,7 +84,25 @@ struct Counters {
   unsigned fate_epoch;  // generation of its tile states
   unsigned de_ticket;   // tile tickets of the force kernel (reset by its last block)
   unsigned de_done;     // blocks of the force kernel that have finished
+  unsigned hist_done;   // blocks of the sort's histogram that have finished
 };
+
+// The commit of update!: the next parity's counters from those of parity p.
+// One thread of one kernel of the step does it, once no other thread still
+// reads the step's births, deaths and flag.
+__device__ __forceinline__ void commit_counters(Counters* C, int p, double dt, bool resort) {
+  C->slots = C->N[p] + C->n_add;
+  C->N[p ^ 1] = C->N[p] + C->n_add - C->n_remove;
+  C->n_add = 0;
+  C->n_remove = 0;
+  C->t[p ^ 1] = C->t[p] + dt;
+  C->step[p ^ 1] = C->step[p] + 1;
+  C->flag[p ^ 1] = 0;
+  C->resort = resort ? 1 : 0;
+  C->events = 0;
+  if (C->list_written) C->list_valid = 1;
+  C->list_written = 0;
+}
 
 template <typename T>
 __device__ __forceinline__ T ld(const T* p) { return __ldg(p); }
@@ -259,6 +277,11 @@ struct ScanArgs {
   int n_tiles;
   Counters* ctr;
   const int* due;                  // skip the scan when *due == 0 (nullptr: always)
+  // the scan also commits the counters of a step of parity p that always
+  // re-sorts, whose force kernel made the histogram
+  int commit = 0;
+  int parity = 0;
+  double dt = 0.0;
 };
 
 // Shared-memory index of cell k of a tile: one padding word per 32 cells, so
@@ -383,6 +406,7 @@ static __global__ void __launch_bounds__(kTile) k_scan_cells(ScanArgs A) {
         A.count[tile_base + k] = 0;
       }
   }
+  if (A.commit && tile == 0 && threadIdx.x == 0) commit_counters(C, A.parity, A.dt, true);
 }
 
 }  // namespace cbm

@@ -63,6 +63,7 @@ struct Params {
   const V4* XS;
   V4* KOUT;
   int no_prune;
+  int hist_in_de;       // the force kernel makes the histogram of the re-sort
   int tiled;            // k_agent_de_tile takes the 3D cell walks of this configuration
   V4* POLD;             // positions at the last Verlet rebuild (slot order)
   int* inv;             // agent index -> slot of A
@@ -1363,6 +1364,25 @@ __global__ void __launch_bounds__(kTile) k_pos32(Params<T> P) {
   }
 }
 
+// In 1D and 2D the force kernel may file the agents in their new cells
+// (2D chemotaxis with 2e5 agents 59.6 -> 55.4 us a step).  In 3D it is short
+// of registers and its warps are few: the histogram in it cost the tiled walk
+// 9 % on the colony of 1e6 agents, and gained nothing on the 256^3 medium.
+template <int D>
+constexpr bool kHistInDE = D < 3;
+template <typename T>
+__device__ __forceinline__ void hist_slot(const Params<T>& P, int s, int c, unsigned lanes);
+
+// Fresh tickets and tile states for the scan that follows a force kernel
+// that makes the sort's histogram.
+template <typename T>
+__device__ __forceinline__ void hist_begin(const Params<T>& P) {
+  if (P.hist_in_de && blockIdx.x == 0 && threadIdx.x == 0) {
+    P.ctr->scan_ticket = 0u;
+    P.ctr->scan_epoch = P.ctr->scan_epoch + 1u;
+  }
+}
+
 // The end of agentStepDE! for slot s once its pair forces are summed in acc:
 // pushing walls, the lagged force, linear drift and chemotaxis, then the
 // integrator (Euler or Euler-Maruyama), the commit of the written slot and
@@ -1439,6 +1459,12 @@ __device__ __forceinline__ void finish_agent(const Params<T>& P, const int s, co
     for (int d = 0; d < D; ++d) xn[d] = xi[d] + dv[d] * P.dt;
   }
   P.PB[s] = from3<T>(xn);
+  if (kHistInDE<D> && P.hist_in_de) {  // no births or deaths, and every step re-sorts
+    const int c = cell_of_pos<T, D>(P, xn);
+    P.s_cell[s] = c;
+    const int n = (int)P.ctr->N[p] - (s & ~31);  // slots of this warp's 32
+    hist_slot(P, s, c, n >= 32 ? kFull : (1u << n) - 1u);
+  }
   P.VB[s] = P.growth ? P.VA[s] + ld(P.G + i) * P.dt : P.VA[s];
   P.IB[s] = i;
   if (is_verlet(P) && !P.ctr->events) {
@@ -1870,6 +1896,7 @@ __global__ void __launch_bounds__(kTile, sizeof(T) == 4 ? 4 : 3) k_agent_de(Para
   if constexpr (D == 3) {
     if (P.tiled && P.neighbors == CBM_NEIGH_CLVD && clvd_walks_cells(P)) return;
   }
+  if constexpr (kHistInDE<D>) hist_begin(P);
   const int N = (int)C->N[P.parity];
   if constexpr (!kPartnerLists<D>) {  // one thread per slot, grid over n_max
     const int slot = (int)blockIdx.x * kTile + (int)threadIdx.x;
@@ -2350,59 +2377,20 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact(Params<T> P) {
 
 // N <- N + NAdd - NRemove, t += dt, step += 1 (update.jl:201-298), and the
 // re-sort decision of computeNeighbors!.  One thread.
-template <typename T>
-__global__ void k_commit(Params<T> P) {
-  Counters* C = P.ctr;
-  const int p = P.parity;
-  C->slots = C->N[p] + C->n_add;
-  C->N[p ^ 1] = C->N[p] + C->n_add - C->n_remove;
-  C->n_add = 0;
-  C->n_remove = 0;
-  C->t[p ^ 1] = C->t[p] + P.dt_time;
-  C->step[p ^ 1] = C->step[p] + 1;
-  C->flag[p ^ 1] = 0;
-  C->resort = (P.neighbors == CBM_NEIGH_CELL_LINKED || C->flag[p]) ? 1 : 0;
-  C->events = 0;
-  if (C->list_written) C->list_valid = 1;
-  C->list_written = 0;
-}
-
 // ---------------------------------------------------------------------------
 // End of step: B -> A.  Without a re-sort the working slots are copied; with
 // one, live working slots are counting-sorted by (cell, agent index) into A
 // (the grid rebuild of computeNeighbors!, neighbors.jl:918-979, and the
 // compaction gather in one pass).
 // ---------------------------------------------------------------------------
-template <typename T, int D>
-__global__ void __launch_bounds__(kTile) k_sort_hist(Params<T> P) {
-  pdl_wait();
-  const Counters* C = P.ctr;
-  const int s = blockIdx.x * kTile + threadIdx.x;
-  const long long slots = C->slots;
-  if (!C->resort) {
-    if (s < slots) {
-      P.PA[s] = P.PB[s];
-      P.VA[s] = P.VB[s];
-      if (P.force_mode == CBM_FORCE_LAGGED) P.FA[s] = P.FB[s];
-    }
-    return;
-  }
-  if (s == 0) {
-    P.ctr->scan_ticket = 0u;  // fresh tickets and tile-state generation for the scan
-    P.ctr->scan_epoch = C->scan_epoch + 1u;
-  }
-  // The lanes of a warp hold consecutive slots, mostly of one cell in a
-  // dense community: the lanes of each cell take their ranks with one atomic
-  // add (any ranks 0 .. count-1 of a cell do, since the placement orders
-  // the cell's agents by index).  Every lane of the warp gets here.
-  int c = -1;
-  if (s < slots && P.IB[s] >= 0) {
-    T x[3];
-    to3<T>(P.PB[s], x);
-    c = cell_of_pos<T, D>(P, x);
-  }
-  if (s < slots) P.s_cell[s] = c;
-  const unsigned peers = __match_any_sync(kFull, c);
+// Cell c of working slot s (-1: dead) and the slot's rank in it.  The lanes
+// of a warp hold consecutive slots, mostly of one cell in a dense community:
+// the lanes of each cell take their ranks with one atomic add (any ranks 0 ..
+// count-1 of a cell do, since the placement orders the cell's agents by
+// index).  Every lane of `lanes` gets here.
+template <typename T>
+__device__ __forceinline__ void hist_slot(const Params<T>& P, int s, int c, unsigned lanes) {
+  const unsigned peers = __match_any_sync(lanes, c);
   if (c >= 0) {
     const int lane = threadIdx.x & 31;
     const int leader = __ffs(peers) - 1;
@@ -2410,6 +2398,47 @@ __global__ void __launch_bounds__(kTile) k_sort_hist(Params<T> P) {
     if (lane == leader) base = atomicAdd(P.cell_count + c, __popc(peers));
     base = __shfl_sync(peers, base, leader);
     P.s_rank[s] = base + __popc(peers & ((1u << lane) - 1u));
+  }
+}
+
+// `commit`: the last block to finish commits the step's counters (the others
+// have read them by then); without it (an upload) they are set already.
+template <typename T, int D>
+__global__ void __launch_bounds__(kTile) k_sort_hist(Params<T> P, int commit) {
+  pdl_wait();
+  Counters* C = P.ctr;
+  const int s = blockIdx.x * kTile + threadIdx.x;
+  const long long slots = commit ? C->N[P.parity] + C->n_add : C->slots;
+  const bool resort =
+      commit ? P.neighbors == CBM_NEIGH_CELL_LINKED || C->flag[P.parity] : C->resort != 0;
+  if (!resort) {
+    if (s < slots) {
+      P.PA[s] = P.PB[s];
+      P.VA[s] = P.VB[s];
+      if (P.force_mode == CBM_FORCE_LAGGED) P.FA[s] = P.FB[s];
+    }
+  } else {
+    if (s == 0) {
+      C->scan_ticket = 0u;  // fresh tickets and tile-state generation for the scan
+      C->scan_epoch = C->scan_epoch + 1u;
+    }
+    int c = -1;
+    if (s < slots && P.IB[s] >= 0) {
+      T x[3];
+      to3<T>(P.PB[s], x);
+      c = cell_of_pos<T, D>(P, x);
+    }
+    if (s < slots) P.s_cell[s] = c;
+    hist_slot(P, s, c, kFull);
+  }
+  if (!commit) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&C->hist_done, 1u) == gridDim.x - 1) {
+      C->hist_done = 0u;
+      commit_counters(C, P.parity, P.dt_time, resort);
+    }
   }
 }
 

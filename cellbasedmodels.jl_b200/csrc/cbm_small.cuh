@@ -12,7 +12,7 @@
 //          positions (the rule's wall reflection computed on the fly), four
 //          lanes an agent, the same sums in the same order as k_agent_de,
 //          into the working set B; then the histogram of the new cells
-//   scan   update!'s counters (k_commit); every block scans the cell counts
+//   scan   update!'s counters; every block scans the cell counts
 //          into shared memory (the cell grid of these communities fits one
 //          block), block 0 stores the offsets, and agent indices are
 //          scattered by (cell, arrival)
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_steps(Params<T> P0, Par
       P.cell_of_slot[ns] = c;
     }
     for (int c = tid; c < n_cells; c += nth) P.cell_count[c] = 0;
-    if (tid == nth - 1) {  // update!'s counters, as k_commit (no births or deaths here)
+    if (tid == nth - 1) {  // update!'s counters, as commit_counters (no births or deaths here)
       C->slots = C->N[p];
       C->N[p ^ 1] = C->N[p];
       C->n_add = 0;
