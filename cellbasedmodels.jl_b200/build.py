@@ -19,6 +19,7 @@ DEPS = SOURCES + [
     os.path.join(HERE, "csrc", "cbm_kernels.cuh"),
     os.path.join(HERE, "csrc", "cbm_common.cuh"),
     os.path.join(HERE, "csrc", "cbm_grid.cuh"),
+    os.path.join(HERE, "csrc", "cbm_pair.cuh"),
     os.path.join(HERE, "csrc", "cbm_small.cuh"),
     os.path.join(HERE, "csrc", "cbm_stencil_vec.cuh"),
     os.path.join(HERE, "csrc", "cbm_tile.cuh"),

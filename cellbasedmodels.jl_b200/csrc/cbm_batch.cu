@@ -27,6 +27,7 @@
 
 #include "../../include/cbm_b200.h"
 #include "cbm_common.cuh"
+#include "cbm_pair.cuh"
 
 using namespace cbm;
 
@@ -323,77 +324,110 @@ __device__ __forceinline__ void list_row_group(const BatchParams& B, const Comm&
   }
 }
 
-// Rebuild step of slot q: the CLVD list row (verletNeighborsCLVD,
-// neighbors.jl:1071-1131 as intended: the 27 cells x fastest, d < list
-// radius) and, in the same pass and the same order, the force.  For fixed
-// (dz, dy) the cells x-1..x+1 are one contiguous run of slots.
+// Four partners of slot q at v, none[u]: no partner.  The branch-free form
+// where it applies, else one by one.
+__device__ __forceinline__ void terms4(const Comm& C, const PairLine<float>& L, const float* xi,
+                                       const float4* v, const bool* none, float* acc) {
+  if (L.mid && pair_terms4_mid<true>(L, xi, v, none, acc)) return;
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+    if (!none[u]) {
+      const float xj[3] = {v[u].x, v[u].y, v[u].z};
+      pair_force(C, xi, xj, acc);
+    }
+}
+
+// Non-rebuild step of slot q: the force over the list row, four entries at a
+// time, the indices of the next four read ahead, summed in list order.
 template <bool SM>
-__device__ __forceinline__ void build_row(const BatchParams& B, const Comm& C, const float4* X,
-                                          const float* sx, const float* sy, const float* sz,
-                                          int q, const float* xi, int* list, int* nbr_n,
-                                          float* acc) {
-  const int n = C.n, M = B.max_nbrs;
+__device__ __forceinline__ void list_row(const BatchParams& B, const Comm& C,
+                                         const PairLine<float>& L, const float4* X,
+                                         const float* sx, const float* sy, const float* sz,
+                                         int q, const float* xi, const int* list, int m,
+                                         float* acc) {
+  const int n = C.n;
+  const int* row = list + q;
+  int j[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) j[u] = u < m ? row[(long long)u * n] : q;
+  for (int k = 0; k < m; k += 4) {
+    float4 v[4];
+    bool none[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      none[u] = k + u >= m;
+      float xj[3];
+      pos_of<SM>(X, sx, sy, sz, j[u], xj);
+      v[u] = make_float4(xj[0], xj[1], xj[2], 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) j[u] = k + 4 + u < m ? row[(long long)(k + 4 + u) * n] : q;
+    terms4(C, L, xi, v, none, acc);
+  }
+}
+
+// The candidates of slot q in walk order, four positions in flight: the 27
+// cells x fastest, where for fixed (dz, dy) the cells x-1..x+1 are one
+// contiguous run of slots.  hit(s, position) for those within the list radius.
+template <bool SM, typename F>
+__device__ __forceinline__ void for_list_radius(const BatchParams& B, const Comm& C,
+                                                const float4* X, const float* sx, const float* sy,
+                                                const float* sz, int q, const float* xi, F&& hit) {
   const int* start = B.cell_start + C.cell_off;
   int q3[3];
   cell_coords<3>(C.nc, cell_of<float, 3>(B.edge, C.lo, C.hi, C.nc, xi), q3);
   const int xa = max(q3[0] - 1, 0), xb = min(q3[0] + 1, C.nc[0] - 1);
-  int m = 0;
-  for (int dz = -1; dz <= 1; ++dz) {
-    const int z = q3[2] + dz;
-    if (z < 0 || z >= C.nc[2]) continue;
-    for (int dy = -1; dy <= 1; ++dy) {
-      const int y = q3[1] + dy;
-      if (y < 0 || y >= C.nc[1]) continue;
-      const int row = (z * C.nc[1] + y) * C.nc[0];
-      const int s1 = start[row + xb + 1];
-      for (int s = start[row + xa]; s < s1; ++s) {
-        if (s == q) continue;
-        float xj[3];
-        pos_of<SM>(X, sx, sy, sz, s, xj);
-        float e = xi[0] - xj[0];
-        float s2 = e * e;
-        e = xi[1] - xj[1];
-        s2 = s2 + e * e;
-        e = xi[2] - xj[2];
-        s2 = s2 + e * e;
-        if (s2 >= B.skin2) continue;
-        if (!(s2 < B.skin2_lo) && !(sqrtf(s2) < B.skin)) continue;
-        if (m < M) list[(long long)m * n + q] = s;
-        ++m;
-        pair_force(C, xi, xj, acc);
+  for (int r = 0; r < 9; ++r) {
+    const int y = q3[1] + r % 3 - 1, z = q3[2] + r / 3 - 1;
+    if (z < 0 || z >= C.nc[2] || y < 0 || y >= C.nc[1]) continue;
+    const int row = (z * C.nc[1] + y) * C.nc[0];
+    const int s1 = start[row + xb + 1];
+    for (int s = start[row + xa]; s < s1; s += 4) {
+      float xj[4][3], s2[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) pos_of<SM>(X, sx, sy, sz, s + u < s1 ? s + u : q, xj[u]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        float e = xi[0] - xj[u][0];
+        s2[u] = e * e;
+        e = xi[1] - xj[u][1];
+        s2[u] = s2[u] + e * e;
+        e = xi[2] - xj[u][2];
+        s2[u] = s2[u] + e * e;
       }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (s + u < s1 && s + u != q && s2[u] < B.skin2 &&
+            (s2[u] < B.skin2_lo || sqrtf(s2[u]) < B.skin))
+          hit(s + u, xj[u]);
     }
   }
-  if (m > M) atomicOr(B.err, kErrNeighborOverflow);
-  nbr_n[q] = m < M ? m : M;
 }
 
-// Non-rebuild step of slot q: the force over the list row, four entries in
-// flight, summed in list order.
+// Rebuild step of slot q: the CLVD list row (verletNeighborsCLVD,
+// neighbors.jl:1071-1131 as intended: d < list radius), then the force over
+// it.  A row that overflows (an error the next synchronising call reports)
+// takes its force from the walk, as the plain path does.
 template <bool SM>
-__device__ __forceinline__ void list_row(const BatchParams& B, const Comm& C, const float4* X,
-                                         const float* sx, const float* sy, const float* sz,
-                                         int q, const float* xi, const int* list,
-                                         const int* nbr_n, float* acc) {
-  const int n = C.n;
-  const int m = nbr_n[q];
-  const int* row = list + q;
-  int k = 0;
-  for (; k + 4 <= m; k += 4) {
-    int j[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) j[u] = row[(long long)(k + u) * n];
-    float xj[4][3];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) pos_of<SM>(X, sx, sy, sz, j[u], xj[u]);
-#pragma unroll
-    for (int u = 0; u < 4; ++u) pair_force(C, xi, xj[u], acc);
+__device__ __forceinline__ void build_row(const BatchParams& B, const Comm& C,
+                                          const PairLine<float>& L, const float4* X,
+                                          const float* sx, const float* sy, const float* sz,
+                                          int q, const float* xi, int* list, int* nbr_n,
+                                          float* acc) {
+  const int n = C.n, M = B.max_nbrs;
+  int m = 0;
+  for_list_radius<SM>(B, C, X, sx, sy, sz, q, xi, [&](int s, const float*) {
+    if (m < M) list[(long long)m * n + q] = s;
+    ++m;
+  });
+  nbr_n[q] = m < M ? m : M;
+  if (m > M) {
+    atomicOr(B.err, kErrNeighborOverflow);
+    for_list_radius<SM>(B, C, X, sx, sy, sz, q, xi,
+                        [&](int, const float* xj) { pair_force(C, xi, xj, acc); });
+    return;
   }
-  for (; k < m; ++k) {
-    float xj[3];
-    pos_of<SM>(X, sx, sy, sz, row[(long long)k * n], xj);
-    pair_force(C, xi, xj, acc);
-  }
+  list_row<SM>(B, C, L, X, sx, sy, sz, q, xi, list, m, acc);
 }
 
 // all requested steps of one community
@@ -407,6 +441,8 @@ __device__ void run_comm(const BatchParams& B, const Comm& C, int ci, int nsteps
   int* list = B.nbr_list + C.off * (long long)B.max_nbrs;
   int* nbr_n = B.nbr_n + C.off;
   const float4* pold = B.pold + C.off;
+  const PairLine<float> line =
+      make_pair_line<float>(C.cut2, C.k_rep, C.r_rep, C.k_att, C.r_att, true);
   if (threadIdx.x == 0) s_flag[0] = s_flag[1] = 0;
   for (int t = 0; t < nsteps; ++t) {
     if (rebuild) {
@@ -432,8 +468,8 @@ __device__ void run_comm(const BatchParams& B, const Comm& C, int ci, int nsteps
       const float xi[3] = {me.x, me.y, me.z};
       float acc[3] = {0.f, 0.f, 0.f};
       if constexpr (L == 1) {
-        if (rebuild) build_row<SM>(B, C, Xc, sx, sy, sz, q, xi, list, nbr_n, acc);
-        else list_row<SM>(B, C, Xc, sx, sy, sz, q, xi, list, nbr_n, acc);
+        if (rebuild) build_row<SM>(B, C, line, Xc, sx, sy, sz, q, xi, list, nbr_n, acc);
+        else list_row<SM>(B, C, line, Xc, sx, sy, sz, q, xi, list, nbr_n[q], acc);
       } else {
         if (rebuild) build_row_group<SM, L>(B, C, Xc, sx, sy, sz, q, xi, list, nbr_n, acc);
         else list_row_group<SM, L>(B, C, Xc, sx, sy, sz, q, xi, list, nbr_n, acc);
@@ -531,6 +567,11 @@ struct cbm_batch {
   int* nbr_n = nullptr;
   int* nbr_list = nullptr;
   int* d_err = nullptr;
+  // exchange with the host: one community's arrays on the device, and a
+  // page-locked ring that uploads go through without waiting
+  float* d_stage = nullptr;
+  float* h_ring = nullptr;
+  size_t ring_bytes = 0, ring_at = 0;
   cbm_batch_tuning tune{256, 2, 0.3, 0.0, 0, 1};
   std::map<int, cudaGraphExec_t> graphs;  // per nsteps
   int n_sm = 148;
@@ -582,6 +623,51 @@ void free_batch(cbm_batch* b) {
   b->cell_allocs.clear();
   if (b->stream) cudaStreamDestroy(b->stream);
   b->stream = nullptr;
+  if (b->h_ring) cudaFreeHost(b->h_ring);
+  b->h_ring = nullptr;
+}
+
+// `bytes` of the ring; when it comes round, the copies out of it are waited for
+int ring_take(cbm_batch* b, size_t bytes, float** out) {
+  bytes = (bytes + 15) & ~(size_t)15;
+  if (b->ring_at + bytes > b->ring_bytes) {
+    BCUDA(b, cudaStreamSynchronize(b->stream));
+    b->ring_at = 0;
+  }
+  *out = b->h_ring + b->ring_at / 4;
+  b->ring_at += bytes;
+  return CBM_OK;
+}
+
+// A community's positions from index-ordered arrays x | y | z (the agent
+// index rides in w); its next step starts with a rebuild.
+__global__ void k_batch_load(const float* src, int n, float4* P, int* parity, int* rebuild,
+                             long long* step, long long step0) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) {
+    *parity = 0;
+    *rebuild = 1;
+    *step = step0;
+  }
+  if (i < n) P[i] = make_float4(src[i], src[n + i], src[2 * n + i], __int_as_float(i));
+}
+
+// The reverse: the step counter (two words), a fault word (zero before) and a
+// pad, then x | y | z in index order.
+__global__ void k_batch_unload(const float4* P0, const float4* P1, const int* parity,
+                               const long long* step, int n, float* dst) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s == 0) *reinterpret_cast<long long*>(dst) = *step;
+  if (s >= n) return;
+  const float4 p = *parity ? P1[s] : P0[s];
+  const int i = agent_index(p);
+  if (i < 0 || i >= n) {
+    atomicOr(reinterpret_cast<int*>(dst) + 2, 1);
+    return;
+  }
+  dst[4 + i] = p.x;
+  dst[4 + n + i] = p.y;
+  dst[4 + 2 * n + i] = p.z;
 }
 
 double list_radius(const cbm_batch* b) { return b->cutoff + b->tune.skin; }
@@ -803,6 +889,15 @@ int cbm_batch_create(cbm_batch** out, const cbm_config* base, int32_t n_comm,
   b->d_order = (int*)balloc(b->allocs, nc * 4, &ok);
   b->d_head = (int*)balloc(b->allocs, 4, &ok);
   b->d_err = (int*)balloc(b->allocs, 4, &ok);
+  size_t most = 0;
+  for (const Comm& C : b->comms) most = std::max(most, (size_t)C.n);
+  const size_t stage = (4 + 3 * most) * 4;
+  b->d_stage = (float*)balloc(b->allocs, stage, &ok);
+  b->ring_bytes = std::max<size_t>(4u << 20, 2 * (stage + 16));
+  if (ok && cudaMallocHost((void**)&b->h_ring, b->ring_bytes) != cudaSuccess) {
+    b->h_ring = nullptr;
+    ok = false;
+  }
   if (!ok) {
     free_batch(b);
     delete b;
@@ -865,22 +960,17 @@ int cbm_batch_upload(cbm_batch* b, int32_t c, const cbm_state_view* h) {
   if (h->N != C.n) return bfail(b, CBM_ERR_ARG, "community %d holds %d agents, got %lld", c, C.n, (long long)h->N);
   if (C.n && (!h->pos[0] || !h->pos[1] || !h->pos[2])) return bfail(b, CBM_ERR_ARG, "positions are NULL");
   cudaSetDevice(b->device);
-  std::vector<float4> packed((size_t)C.n);
-  const float* x = (const float*)h->pos[0];
-  const float* y = (const float*)h->pos[1];
-  const float* z = (const float*)h->pos[2];
-  for (int i = 0; i < C.n; ++i) {
-    float w;
-    memcpy(&w, &i, sizeof w);  // the agent index rides in w
-    packed[(size_t)i] = make_float4(x[i], y[i], z[i], w);
-  }
-  BCUDA(b, cudaStreamSynchronize(b->stream));
-  if (C.n) BCUDA(b, cudaMemcpy(b->P[0] + C.off, packed.data(), (size_t)C.n * 16, cudaMemcpyHostToDevice));
-  int zero = 0, one = 1;
-  long long st = h->step;
-  BCUDA(b, cudaMemcpy(b->parity + c, &zero, 4, cudaMemcpyHostToDevice));
-  BCUDA(b, cudaMemcpy(b->rebuild + c, &one, 4, cudaMemcpyHostToDevice));
-  BCUDA(b, cudaMemcpy(b->step + c, &st, 8, cudaMemcpyHostToDevice));
+  // the caller's arrays into the pinned ring, one copy and one kernel on the
+  // stream: no wait, unless the ring comes round
+  const size_t nb = (size_t)C.n * 4;
+  float* host = nullptr;
+  if (int rc = ring_take(b, 3 * nb, &host)) return rc;
+  for (int d = 0; d < 3; ++d)
+    if (C.n) memcpy(host + (size_t)d * C.n, h->pos[d], nb);
+  if (C.n) BCUDA(b, cudaMemcpyAsync(b->d_stage, host, 3 * nb, cudaMemcpyHostToDevice, b->stream));
+  k_batch_load<<<(std::max(C.n, 1) + 255) / 256, 256, 0, b->stream>>>(
+      b->d_stage, C.n, b->P[0] + C.off, b->parity + c, b->rebuild + c, b->step + c, h->step);
+  BCUDA(b, cudaGetLastError());
   return CBM_OK;
 }
 
@@ -889,26 +979,25 @@ int cbm_batch_download(cbm_batch* b, int32_t c, cbm_state_view* h) {
   const Comm& C = b->comms[(size_t)c];
   if (h->capacity < C.n) return bfail(b, CBM_ERR_ARG, "host capacity too small");
   cudaSetDevice(b->device);
+  // slot order -> index order on the device, then one copy: the step counter
+  // and a fault word, x, y, z
+  const size_t words = 4 + 3 * (size_t)C.n;
+  float* host = nullptr;
+  if (int rc = ring_take(b, words * 4, &host)) return rc;
+  BCUDA(b, cudaMemsetAsync(b->d_stage, 0, 16, b->stream));
+  k_batch_unload<<<(std::max(C.n, 1) + 255) / 256, 256, 0, b->stream>>>(
+      b->P[0] + C.off, b->P[1] + C.off, b->parity + c, b->step + c, C.n, b->d_stage);
+  BCUDA(b, cudaGetLastError());
+  BCUDA(b, cudaMemcpyAsync(host, b->d_stage, words * 4, cudaMemcpyDeviceToHost, b->stream));
   BCUDA(b, cudaStreamSynchronize(b->stream));
-  int par = 0;
+  b->ring_at = 0;
   long long st = 0;
-  BCUDA(b, cudaMemcpy(&par, b->parity + c, 4, cudaMemcpyDeviceToHost));
-  BCUDA(b, cudaMemcpy(&st, b->step + c, 8, cudaMemcpyDeviceToHost));
-  std::vector<float4> packed((size_t)C.n);
-  if (C.n) BCUDA(b, cudaMemcpy(packed.data(), b->P[par] + C.off, (size_t)C.n * 16, cudaMemcpyDeviceToHost));
-  float* x = (float*)h->pos[0];
-  float* y = (float*)h->pos[1];
-  float* z = (float*)h->pos[2];
-  // slot order -> index order
-  for (int s = 0; s < C.n; ++s) {
-    const float4& p = packed[(size_t)s];
-    int i;
-    memcpy(&i, &p.w, sizeof i);
-    if (i < 0 || i >= C.n) return bfail(b, CBM_ERR_CUDA, "community %d: corrupt agent index", c);
-    if (x) x[i] = p.x;
-    if (y) y[i] = p.y;
-    if (z) z[i] = p.z;
-  }
+  int bad = 0;
+  memcpy(&st, host, 8);
+  memcpy(&bad, host + 2, 4);
+  if (bad) return bfail(b, CBM_ERR_CUDA, "community %d: corrupt agent index", c);
+  for (int d = 0; d < 3; ++d)
+    if (h->pos[d] && C.n) memcpy(h->pos[d], host + 4 + (size_t)d * C.n, (size_t)C.n * 4);
   h->N = C.n;
   h->step = st;
   h->t = (double)st * b->base.dt;

@@ -25,6 +25,7 @@
 #include <type_traits>
 
 #include "cbm_common.cuh"
+#include "cbm_pair.cuh"
 
 namespace cbm {
 
@@ -1185,44 +1186,6 @@ __global__ void __launch_bounds__(kTile) k_agent_fate(Params<T> P) {
 // agentStepDE!: fused neighbor force + Euler / EM update, one thread per slot
 // (src/integrators.jl:465-505,683-734, functionDE.jl:13-117)
 // ---------------------------------------------------------------------------
-// Packed pairs of float operations (sm_100 f32x2): one instruction, and per
-// element the same IEEE rounding as the scalar operation.
-__device__ __forceinline__ float2 f2_sub(float2 a, float2 b) {
-  unsigned long long r;
-  asm("sub.rn.f32x2 %0, %1, %2;"
-      : "=l"(r)
-      : "l"(*reinterpret_cast<unsigned long long*>(&a)),
-        "l"(*reinterpret_cast<unsigned long long*>(&b)));
-  return *reinterpret_cast<float2*>(&r);
-}
-__device__ __forceinline__ float2 f2_mul(float2 a, float2 b) {
-  unsigned long long r;
-  asm("mul.rn.f32x2 %0, %1, %2;"
-      : "=l"(r)
-      : "l"(*reinterpret_cast<unsigned long long*>(&a)),
-        "l"(*reinterpret_cast<unsigned long long*>(&b)));
-  return *reinterpret_cast<float2*>(&r);
-}
-
-__device__ __forceinline__ float2 f2_add(float2 a, float2 b) {
-  unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;"
-      : "=l"(r)
-      : "l"(*reinterpret_cast<unsigned long long*>(&a)),
-        "l"(*reinterpret_cast<unsigned long long*>(&b)));
-  return *reinterpret_cast<float2*>(&r);
-}
-
-__device__ __forceinline__ float2 f2_fma(float2 a, float2 b, float2 c) {
-  unsigned long long r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(r)
-      : "l"(*reinterpret_cast<unsigned long long*>(&a)),
-        "l"(*reinterpret_cast<unsigned long long*>(&b)),
-        "l"(*reinterpret_cast<unsigned long long*>(&c)));
-  return *reinterpret_cast<float2*>(&r);
-}
-
 // e = xi - xj and its squared norm, in the reference's order
 // ((e0 e0 + e1 e1) + e2 e2); in Float32 the x and y halves are packed pairs.
 template <typename T, int D>

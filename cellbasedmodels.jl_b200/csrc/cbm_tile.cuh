@@ -125,78 +125,23 @@ __device__ __forceinline__ uint4 tile_row(float x, float y, float z, float c, bo
   return r;
 }
 
-// The pair term in a form without branches: base and stiffness are selected,
-// and every pair beyond the cutoff, or the agent itself, adds a zero.  In
-// Float32 all of it is kept negated (-d^2, -d), which leaves no negations
-// between the packed operations.
-template <typename T>
-struct PairLine {
-  T nfar2, nreach, nrrep, krep, katt, rrep, abase;
-  bool mid;  // the stiffnesses are far from the ends of the exponent range
-};
+// The branch-free form's coefficients (cbm_pair.cuh) of the model.
 template <typename T>
 __device__ __forceinline__ PairLine<T> pair_line(const Params<T>& P) {
-  const bool rep = P.att_form == CBM_ATT_FROM_REP;
-  auto mid = [](T k) { return k == (T)0 || (fabs(k) > (T)1e-12 && fabs(k) < (T)1e12); };
-  // -(a (d - r)) and a (r - d) are the same number; so are -(a (c - d)) and
-  // (-a) (c - d).  A squared distance of cut2 is a distance >= the cutoff.
-  return PairLine<T>{-P.cut2, -(P.r_rep > P.r_att ? P.r_rep : P.r_att), -P.r_rep, P.k_rep,
-                     rep ? P.k_att : -P.k_att, P.r_rep, rep ? P.r_rep : P.r_att,
-                     mid(P.k_rep) && mid(P.k_att)};
+  return make_pair_line<T>(P.cut2, P.k_rep, P.r_rep, P.k_att, P.r_att,
+                           P.att_form == CBM_ATT_FROM_REP);
 }
 
 // The terms of four partners at positions v, added to acc in order; an entry
 // that is the agent itself adds nothing.  `plain`: the positions are within
-// kTileReach of one another and L.mid holds.  Square root and quotient are
-// sqrt_mid and div_mid on pairs of values.
+// kTileReach of one another and L.mid holds.
 template <typename T>
 __device__ __forceinline__ void pair_terms4(const PairCoef<T>& c, const PairLine<T>& L, bool plain,
                                             const T* xi, const typename V4T<T>::type* v, int s,
                                             const int* qq, T* acc) {
   if constexpr (std::is_same<T, float>::value) {
-    const float2 ixy = make_float2(xi[0], xi[1]);
-    float2 exy[4], n2[2];
-    float ez[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      exy[u] = f2_sub(ixy, make_float2(v[u].x, v[u].y));
-      ez[u] = xi[2] - v[u].z;
-      const float2 q = f2_mul(exy[u], exy[u]);
-      const float n = (-q.x - q.y) - ez[u] * ez[u];
-      (u & 1 ? n2[u >> 1].y : n2[u >> 1].x) = qq[u] == s ? L.nfar2 : n;
-    }
-    // coincident agents take the general form
-    if (plain && fmaxf(fmaxf(n2[0].x, n2[0].y), fmaxf(n2[1].x, n2[1].y)) < -1e-12f) {
-#pragma unroll
-      for (int p = 0; p < 2; ++p) {
-        const float2 x = n2[p], half = make_float2(0.5f, 0.5f);
-        float2 y;
-        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(-x.x));
-        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(-x.y));
-        float2 g = f2_mul(x, y), h = f2_mul(half, y);
-        float2 r = f2_fma(g, h, half);
-        g = f2_fma(g, r, g);
-        h = f2_fma(h, r, h);
-        const float2 d = f2_fma(f2_fma(g, g, x), h, g);  // minus the distances
-        const bool r0 = d.x > L.nrrep, r1 = d.y > L.nrrep;
-        const float2 k = make_float2(r0 ? L.krep : L.katt, r1 ? L.krep : L.katt);
-        const float2 b = make_float2(r0 ? L.rrep : L.abase, r1 ? L.rrep : L.abase);
-        const float2 F = f2_mul(k, f2_add(b, d));
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(-d.x));
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(-d.y));
-        y = f2_fma(y, f2_fma(d, y, make_float2(1.f, 1.f)), y);
-        float2 q = f2_mul(F, y);
-        q = f2_fma(f2_fma(d, q, F), y, q);
-        const float c0 = d.x > L.nreach ? q.x : 0.f, c1 = d.y > L.nreach ? q.y : 0.f;
-        const float2 t0 = f2_mul(make_float2(c0, c0), exy[2 * p]);
-        const float2 t1 = f2_mul(make_float2(c1, c1), exy[2 * p + 1]);
-        // scalar sums: a packed product and a packed sum came out fused
-        acc[0] = (acc[0] + t0.x) + t1.x;
-        acc[1] = (acc[1] + t0.y) + t1.y;
-        acc[2] = (acc[2] + c0 * ez[2 * p]) + c1 * ez[2 * p + 1];
-      }
-      return;
-    }
+    const bool none[4] = {qq[0] == s, qq[1] == s, qq[2] == s, qq[3] == s};
+    if (plain && pair_terms4_mid<false>(L, xi, v, none, acc)) return;
   }
   if constexpr (std::is_same<T, double>::value) {
     double e[4][3], n2[4];
