@@ -20,19 +20,23 @@
 // program compute.
 //
 // Memory: checkpoints every `checkpoint_every` steps; a segment is recomputed
-// from its checkpoint, keeping its states, cell grids and interacting pairs,
-// and then swept backwards, so long trajectories need O(T/K + K) states
-// instead of O(T).
+// from its checkpoint, keeping each step's slot positions and interacting
+// pairs, and then swept backwards, so long trajectories need O(T/K + K)
+// states instead of O(T).  The last segment's are kept by the forward sweep
+// itself, into the same buffers, and not computed twice.
 //
-// Layout and launches.  Each step's grid (counting sort by cell, ascending
-// index inside a cell) is followed by a gather of the positions into slot
-// order (double4/float4 with the agent index in w), so a thread walks its 27
-// cells as 9 contiguous slot runs, in the reference's order.  The recompute
-// pass records, per slot, the partner slots that carry a force term; the
-// backward step visits only those pairs.  All buffers of a shape (n, steps,
-// checkpoint interval) are kept, and the whole device part of a run is one
-// CUDA graph replayed by later runs of the same shape; host copies of the
-// inputs and results stay outside the graph.
+// Layout and launches.  States are double4/float4 in index order.  A step is
+// four kernels: the scan of the cell counts, the scatter, the placement of
+// the positions in slot order (cells x fastest, ascending index inside a
+// cell; the agent index rides in w), and the Euler step by tiles of 32 slots
+// (cbm_tile.cuh), which also files the new positions in their cells.  They
+// follow one another by programmatic launches.  A backward step is one kernel
+// over the recorded pairs, four lanes an agent (at 65536 agents one lane
+// leaves 3.5 warps a scheduler, each in a serial chain); it reads the
+// partners' lambda by their index.  All buffers of a shape (n, steps, checkpoint interval) are
+// kept, and the whole device part of a run is one CUDA graph replayed by
+// later runs of the same shape; host copies of the inputs and results stay
+// outside the graph.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -44,7 +48,7 @@
 #include <vector>
 
 #include "../../include/cbm_b200.h"
-#include "cbm_grid.cuh"
+#include "cbm_tile.cuh"
 
 using namespace cbm;
 
@@ -68,14 +72,22 @@ struct AV4<double> {
 template <typename T>
 struct AdjParams {
   using V4 = typename AV4<T>::type;
-  T* xn[3];             // x_{n+1}, index order (forward)
-  const V4* xs;         // x_n in slot order, w = agent index
-  const V4* ls;         // lambda_{n+1} in slot order (backward)
-  T* lam_out[3];        // lambda_n, index order (backward)
+  const V4* x;          // state, index order
+  V4* xn;               // x_{n+1}, index order (forward)
+  V4* xs;               // x_n in slot order, w = agent index
+  const V4* lam;        // lambda_{n+1}, index order (backward)
+  V4* lam_out;          // lambda_n
+  int* cell_count;
   const int* cell_start;
-  int* pair_n;          // per slot: partners with a force term (recompute, backward)
+  int* agent_cell;      // per agent: cell of the state filed last, rank in it
+  int* agent_rank;
+  int* cell_tmp;        // agents by cell, in arrival order
+  int* cell_of_slot;    // cell of each slot of xs
+  int* pair_n;          // per slot: partners with a force term (recorded steps), or null
   int* pair_list;       // entry k of slot s at k * n + s: the partner's slot
   int cap;
+  bool file;            // the step files x_{n+1} in its cells
+  bool mid;             // the stiffnesses suit sqrt_mid and div_mid
   double* gpart;        // per block: running dL/dtheta partials (3 per block)
   Counters* ctr;
   int n;
@@ -85,126 +97,200 @@ struct AdjParams {
   T dt, k, a, rho, ratt, cut2;
 };
 
-// x (index order) gathered into slot order, agent index in w
+constexpr int kLanes = 4;                // lanes an agent (backward)
+constexpr int kSlots = kTile / kLanes;   // slots a block
+
+// fresh tickets and tile states for the scan that follows
 template <typename T>
-__global__ void __launch_bounds__(kTile) k_adj_gather(const T* x0, const T* x1, const T* x2,
-                                                      const int* agents, typename AV4<T>::type* out,
-                                                      int n) {
-  const int s = blockIdx.x * kTile + threadIdx.x;
-  if (s >= n) return;
-  const int j = agents[s];
-  typename AV4<T>::type v;
-  v.x = x0[j];
-  v.y = x1[j];
-  v.z = x2[j];
-  v.w = AV4<T>::enc(j);
-  out[s] = v;
+__device__ __forceinline__ void adj_scan_begin(const AdjParams<T>& A) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    A.ctr->scan_ticket = 0u;
+    A.ctr->scan_epoch = A.ctr->scan_epoch + 1u;
+  }
 }
 
-// forward Euler step of the agent in slot s: the reference's expression
-// order, cells x fastest, ascending index inside a cell (the plain path's
-// CellLinked sums).  With LIST, the slots of the partners that carry a
-// force term are recorded in order for the backward step.
-template <typename T, bool LIST>
-__global__ void __launch_bounds__(kTile) k_adj_forward(AdjParams<T> A) {
-  const int s = blockIdx.x * kTile + threadIdx.x;
-  if (s >= A.n) return;
-  const typename AV4<T>::type me = A.xs[s];
-  const int i = AV4<T>::dec(me.w);
+// agent i at v filed in its cell (assignCells, neighbors.jl:763-821)
+template <typename T>
+__device__ __forceinline__ void adj_file(const AdjParams<T>& A, int i, const T* x) {
+  const int c = cell_of<T, 3>(A.edge, A.lo, A.hi, A.nc, x);
+  A.agent_cell[i] = c;
+  A.agent_rank[i] = atomicAdd(A.cell_count + c, 1);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kTile) k_adj_file(AdjParams<T> A) {
+  pdl_wait();
+  adj_scan_begin(A);
+  const int i = blockIdx.x * kTile + threadIdx.x;
+  if (i >= A.n) return;
+  const typename AV4<T>::type v = A.x[i];
+  const T x[3] = {v.x, v.y, v.z};
+  adj_file(A, i, x);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kTile) k_adj_scatter(AdjParams<T> A) {
+  pdl_wait();
+  const int i = blockIdx.x * kTile + threadIdx.x;
+  if (i >= A.n) return;
+  A.cell_tmp[A.cell_start[A.agent_cell[i]] + A.agent_rank[i]] = i;
+}
+
+// rank among the cell's agents with a smaller index (neighbors.jl:851-862)
+template <typename T>
+__global__ void __launch_bounds__(kTile) k_adj_place(AdjParams<T> A) {
+  pdl_wait();
+  const int i = blockIdx.x * kTile + threadIdx.x;
+  if (i >= A.n) return;
+  typename AV4<T>::type v = A.x[i];
+  const int c = A.agent_cell[i];
+  const int s0 = A.cell_start[c], s1 = A.cell_start[c + 1];
+  int r = 0;
+  for (int s = s0; s < s1; ++s) r += A.cell_tmp[s] < i;
+  v.w = AV4<T>::enc(i);
+  A.xs[s0 + r] = v;
+  A.cell_of_slot[s0 + r] = c;
+}
+
+// three index-ordered arrays <-> states
+template <typename T>
+__global__ void __launch_bounds__(kTile) k_adj_pack(const T* x0, const T* x1, const T* x2,
+                                                    typename AV4<T>::type* out, int n) {
+  const int i = blockIdx.x * kTile + threadIdx.x;
+  if (i >= n) return;
+  typename AV4<T>::type v;
+  v.x = x0[i];
+  v.y = x1[i];
+  v.z = x2[i];
+  v.w = (T)0;
+  out[i] = v;
+}
+template <typename T>
+__global__ void __launch_bounds__(kTile) k_adj_unpack(const typename AV4<T>::type* in, T* x0, T* x1,
+                                                      T* x2, int n) {
+  const int i = blockIdx.x * kTile + threadIdx.x;
+  if (i >= n) return;
+  const typename AV4<T>::type v = in[i];
+  x0[i] = v.x;
+  x1[i] = v.y;
+  x2[i] = v.z;
+}
+
+// a checkpoint (a kernel, so that the step after it may launch programmatically)
+template <typename T>
+__global__ void __launch_bounds__(kTile) k_adj_keep(const typename AV4<T>::type* x,
+                                                    typename AV4<T>::type* out, int n) {
+  const int i = blockIdx.x * kTile + threadIdx.x;
+  if (i < n) out[i] = x[i];
+}
+
+// square root and quotient of the pair terms: the branch-free forms where
+// they are exact (every recorded pair is closer than the cutoff)
+template <typename T>
+__device__ __forceinline__ T adj_sqrt(bool mid, T x, T* inv) {
+  if (mid) {
+    if constexpr (sizeof(T) == 8) return sqrt_mid(x, inv);
+    else return sqrt_mid(x);
+  }
+  return sqrt(x);
+}
+template <typename T>
+__device__ __forceinline__ T adj_div(bool mid, T a, T b, T inv) {
+  if (mid) {
+    if constexpr (sizeof(T) == 8) return div_mid(a, b, inv);
+    else return div_mid(a, b);
+  }
+  return a / b;
+}
+
+template <typename T>
+__device__ __forceinline__ T adj_diff(const T* xi, const typename AV4<T>::type& o, T* e) {
+  e[0] = xi[0] - o.x;
+  T s2 = e[0] * e[0];
+  e[1] = xi[1] - o.y;
+  s2 = s2 + e[1] * e[1];
+  e[2] = xi[2] - o.z;
+  return s2 + e[2] * e[2];
+}
+
+// forward Euler step by tiles of 32 slots (cbm_tile.cuh): the reference's
+// expression order, cells x fastest, ascending index inside a cell (the plain
+// path's CellLinked sums).  A recorded step keeps the slots of the partners
+// that carry a force term, in that order.
+template <typename T>
+__global__ void __launch_bounds__(32, kTileWarps) k_adj_step(Params<T> P, AdjParams<T> A) {
+  __shared__ TileSmem S;
+  pdl_wait();
+  if (A.file) adj_scan_begin(A);
+  tile_begin(S);
+  const int s0 = blockIdx.x * 32, s = s0 + (int)threadIdx.x;
+  if (s0 >= A.n) return;
+  const typename AV4<T>::type me = A.xs[s < A.n ? s : A.n - 1];
   const T xi[3] = {me.x, me.y, me.z};
-  int q[3];
-  cell_coords<3>(A.nc, cell_of<T, 3>(A.edge, A.lo, A.hi, A.nc, xi), q);
-  const int xa = max(q[0] - 1, 0), xb = min(q[0] + 1, A.nc[0] - 1);
   T acc[3] = {(T)0, (T)0, (T)0};
   int m = 0;
-  for (int dz = -1; dz <= 1; ++dz) {
-    const int z = q[2] + dz;
-    if (z < 0 || z >= A.nc[2]) continue;
-    for (int dy = -1; dy <= 1; ++dy) {
-      const int y = q[1] + dy;
-      if (y < 0 || y >= A.nc[1]) continue;
-      const int row = (z * A.nc[1] + y) * A.nc[0];
-      const int t1 = A.cell_start[row + xb + 1];
-      for (int t = A.cell_start[row + xa]; t < t1; ++t) {
-        if (t == s) continue;
-        const typename AV4<T>::type o = A.xs[t];
-        T e[3];
-        e[0] = xi[0] - o.x;
-        T s2 = e[0] * e[0];
-        e[1] = xi[1] - o.y;
-        s2 = s2 + e[1] * e[1];
-        e[2] = xi[2] - o.z;
-        s2 = s2 + e[2] * e[2];
-        if (s2 >= A.cut2) continue;
-        const T dd = sqrt(s2);
-        T F;
-        if (dd < A.rho) F = A.k * (A.rho - dd);
-        else if (dd < A.ratt) F = -(A.a * (dd - A.rho));
-        else continue;
-        const T sc = F / dd;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) acc[d] = acc[d] + sc * e[d];
-        if (LIST) {
-          if (m < A.cap) A.pair_list[(long long)m * A.n + s] = t;
-          ++m;
-        }
-      }
-    }
-  }
-  if (LIST) {
+  int* const list = A.pair_n ? A.pair_list + s : nullptr;
+  tile_forces<T>(P, S, A.n, s0, xi, acc, [&](int q) {
+    if (list && m < A.cap) list[(long long)m * A.n] = q;
+    ++m;
+  });
+  if (s >= A.n) return;
+  if (A.pair_n) {
     A.pair_n[s] = m < A.cap ? m : A.cap;
     if (m > A.cap) atomicOr(&A.ctr->err, kErrNeighborOverflow);
   }
-#pragma unroll
-  for (int d = 0; d < 3; ++d) A.xn[d][i] = xi[d] + acc[d] * A.dt;
+  const int i = AV4<T>::dec(me.w);
+  const T xn[3] = {xi[0] + acc[0] * A.dt, xi[1] + acc[1] * A.dt, xi[2] + acc[2] * A.dt};
+  typename AV4<T>::type out;
+  out.x = xn[0];
+  out.y = xn[1];
+  out.z = xn[2];
+  out.w = (T)0;
+  A.xn[i] = out;
+  if (A.file) adj_file(A, i, xn);
 }
 
 // one backward step at state x_n: lambda_n from lambda_{n+1} over the pairs
-// recorded by the recompute pass, and this step's dL/dtheta terms added to
-// the block's running partial sums
+// recorded by the forward step, and this step's dL/dtheta terms added to the
+// block's running partial sums.  The lanes of an agent take its pairs in turn
+// and their sums meet in a fixed tree.
 template <typename T>
 __global__ void __launch_bounds__(kTile) k_adj_backward(AdjParams<T> A) {
-  __shared__ double red[3][kTile];
-  const int s = blockIdx.x * kTile + threadIdx.x;
-  double g[3] = {0.0, 0.0, 0.0};
+  __shared__ double red[3][kTile / 32];
+  pdl_wait();
+  const int s = blockIdx.x * kSlots + (int)threadIdx.x / kLanes;
+  const int lane = threadIdx.x & 31, u = lane & (kLanes - 1);
+  T adj[3] = {(T)0, (T)0, (T)0};
+  T th[3] = {(T)0, (T)0, (T)0};  // k, a, rho
+  T li[3] = {(T)0, (T)0, (T)0};
+  int i = 0;
   if (s < A.n) {
     const typename AV4<T>::type me = A.xs[s];
-    const typename AV4<T>::type lm = A.ls[s];
-    const int i = AV4<T>::dec(me.w);
+    i = AV4<T>::dec(me.w);
+    const typename AV4<T>::type lm = A.lam[i];
     const T xi[3] = {me.x, me.y, me.z};
-    const T li[3] = {lm.x, lm.y, lm.z};
-    T adj[3] = {(T)0, (T)0, (T)0};
-    T gk = (T)0, ga = (T)0, gr = (T)0;
+    li[0] = lm.x;
+    li[1] = lm.y;
+    li[2] = lm.z;
     const int m = A.pair_n[s];
-    for (int kk = 0; kk < m; ++kk) {
-      const int t = A.pair_list[(long long)kk * A.n + s];
+    const int* const list = A.pair_list + s;
+    int t = u < m ? list[(long long)u * A.n] : s;
+    for (int kk = u; kk < m; kk += kLanes) {
       const typename AV4<T>::type o = A.xs[t];
-      const typename AV4<T>::type lo = A.ls[t];
+      if (kk + kLanes < m) t = list[(long long)(kk + kLanes) * A.n];
+      const typename AV4<T>::type lo = A.lam[AV4<T>::dec(o.w)];
       T r[3];
-      r[0] = xi[0] - o.x;
-      T s2 = r[0] * r[0];
-      r[1] = xi[1] - o.y;
-      s2 = s2 + r[1] * r[1];
-      r[2] = xi[2] - o.z;
-      s2 = s2 + r[2] * r[2];
-      const T dd = sqrt(s2);  // every recorded pair has dd < r_att
-      T F, Fp, dk, da, drho;
-      if (dd < A.rho) {
-        F = A.k * (A.rho - dd);
-        Fp = -A.k;
-        dk = A.rho - dd;
-        da = (T)0;
-        drho = A.k;
-      } else {
-        F = -(A.a * (dd - A.rho));
-        Fp = -A.a;
-        dk = (T)0;
-        da = -(dd - A.rho);
-        drho = A.a;
-      }
-      const T inv = (T)1 / dd;
+      const T s2 = adj_diff(xi, o, r);
+      const bool mid = A.mid && s2 > (T)1e-12;
+      T inv0 = (T)0;
+      const T dd = adj_sqrt(mid, s2, &inv0);  // every recorded pair has dd < r_att
+      const bool rep = dd < A.rho;
+      const T kk_ = rep ? A.k : A.a;
+      const T gap = A.rho - dd;
+      const T F = kk_ * gap;
+      const T inv = adj_div(mid, (T)1, dd, inv0);
       const T sc = F * inv;
-      const T c = (Fp * dd - F) * inv * inv * inv;
+      const T c = (-kk_ * dd - F) * inv * inv * inv;
       const T dl[3] = {li[0] - lo.x, li[1] - lo.y, li[2] - lo.z};
       T rdl = (T)0, rli = (T)0;
 #pragma unroll
@@ -214,48 +300,65 @@ __global__ void __launch_bounds__(kTile) k_adj_backward(AdjParams<T> A) {
       }
 #pragma unroll
       for (int d = 0; d < 3; ++d) adj[d] += sc * dl[d] + c * rdl * r[d];
-      gk += dk * inv * rli;
-      ga += da * inv * rli;
-      gr += drho * inv * rli;
+      const T w = inv * rli;
+      th[0] += rep ? gap * w : (T)0;
+      th[1] += rep ? (T)0 : gap * w;
+      th[2] += kk_ * w;
     }
+  }
 #pragma unroll
-    for (int d = 0; d < 3; ++d) A.lam_out[d][i] = li[d] + A.dt * adj[d];
-    g[0] = (double)(A.dt * gk);
-    g[1] = (double)(A.dt * ga);
-    g[2] = (double)(A.dt * gr);
+  for (int o = 1; o < kLanes; o <<= 1)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      adj[d] += __shfl_xor_sync(kFull, adj[d], o);
+      th[d] += __shfl_xor_sync(kFull, th[d], o);
+    }
+  if (s < A.n && u == 0) {
+    typename AV4<T>::type out;
+    out.x = li[0] + A.dt * adj[0];
+    out.y = li[1] + A.dt * adj[1];
+    out.z = li[2] + A.dt * adj[2];
+    out.w = (T)0;
+    A.lam_out[i] = out;
   }
   // deterministic block sum (fixed tree), added to this block's running sum
 #pragma unroll
-  for (int q = 0; q < 3; ++q) red[q][threadIdx.x] = g[q];
-  __syncthreads();
-  for (int o = kTile / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o)
+  for (int q = 0; q < 3; ++q) {
+    double g = (double)(A.dt * th[q]);
 #pragma unroll
-      for (int q = 0; q < 3; ++q) red[q][threadIdx.x] += red[q][threadIdx.x + o];
-    __syncthreads();
+    for (int o = kLanes; o < 32; o <<= 1) g += __shfl_xor_sync(kFull, g, o);
+    if (lane == 0) red[q][threadIdx.x >> 5] = g;
   }
-  if (threadIdx.x < 3) A.gpart[blockIdx.x * 3 + threadIdx.x] += red[threadIdx.x][0];
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    double g = 0.0;
+#pragma unroll
+    for (int w = 0; w < kTile / 32; ++w) g += red[threadIdx.x][w];
+    A.gpart[blockIdx.x * 3 + threadIdx.x] += g;
+  }
 }
 
 // lambda_T = 2 (x_T - x*) / (3N) and per-block partial sums of the loss
 template <typename T>
-__global__ void __launch_bounds__(kTile) k_adj_loss(const T* x0, const T* x1, const T* x2,
-                                                    const T* tgt0, const T* tgt1, const T* tgt2,
-                                                    T* l0, T* l1, T* l2, int n, double* lpart) {
+__global__ void __launch_bounds__(kTile) k_adj_loss(const typename AV4<T>::type* x, const T* tgt0,
+                                                    const T* tgt1, const T* tgt2,
+                                                    typename AV4<T>::type* lam, int n,
+                                                    double* lpart) {
   __shared__ double red[kTile];
   const int i = blockIdx.x * kTile + threadIdx.x;
-  const T* x[3] = {x0, x1, x2};
-  const T* tg[3] = {tgt0, tgt1, tgt2};
-  T* lo[3] = {l0, l1, l2};
   double l = 0.0;
   if (i < n) {
     const T inv3n = (T)2 / (T)(3.0 * (double)n);
+    const typename AV4<T>::type v = x[i];
+    const T e[3] = {v.x - tgt0[i], v.y - tgt1[i], v.z - tgt2[i]};
+    typename AV4<T>::type o;
+    o.x = inv3n * e[0];
+    o.y = inv3n * e[1];
+    o.z = inv3n * e[2];
+    o.w = (T)0;
+    lam[i] = o;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const T e = x[d][i] - tg[d][i];
-      lo[d][i] = inv3n * e;
-      l += (double)e * (double)e;
-    }
+    for (int d = 0; d < 3; ++d) l += (double)e[d] * (double)e[d];
   }
   red[threadIdx.x] = l;
   __syncthreads();
@@ -278,7 +381,8 @@ struct Plan {
   void* out_dx0[3] = {}; // lambda_0
   double* gpart = nullptr;
   double* lpart = nullptr;
-  int blocks = 1;
+  int blocks = 1;        // of one thread an agent (lpart)
+  int step_blocks = 1;   // of kLanes threads an agent (gpart)
   void release() {
     if (graph) cudaGraphExecDestroy(graph);
     graph = nullptr;
@@ -308,6 +412,7 @@ struct cbm_adjoint {
   int* agent_cell = nullptr;
   int* agent_rank = nullptr;
   int* cell_tmp = nullptr;
+  int* cell_of_slot = nullptr;
   Counters* ctr = nullptr;
   Plan plan[2];          // [0] forward only, [1] forward + backward
 };
@@ -335,45 +440,6 @@ int afail(cbm_adjoint* a, int code, const char* fmt, ...) {
   } while (0)
 
 template <typename T>
-GridParams<T> grid_params(cbm_adjoint* a, const T* const* x, int n, int* cell_start,
-                          int* cell_agents) {
-  GridParams<T> G;
-  memset(&G, 0, sizeof G);
-  for (int d = 0; d < 3; ++d) {
-    G.pos[d] = x[d];
-    G.box_lo[d] = (T)a->cfg.box_lo[d];
-    G.box_hi[d] = (T)a->cfg.box_hi[d];
-    G.n_cells_d[d] = a->nc[d];
-  }
-  G.n = n;
-  G.edge = (T)a->cfg.cell_edge;
-  G.n_cells = a->n_cells;
-  G.n_scan_tiles = a->n_tiles;
-  G.ctr = a->ctr;
-  G.cell_count = a->cell_count;
-  G.cell_start = cell_start;
-  G.scan_state = a->scan_state;
-  G.agent_cell = a->agent_cell;
-  G.agent_rank = a->agent_rank;
-  G.cell_tmp = a->cell_tmp;
-  G.cell_agents = cell_agents;
-  return G;
-}
-
-// grid of state x (index order) and its positions in slot order
-template <typename T>
-void build_grid(cbm_adjoint* a, T* const* x, int n, int* cell_start, int* cell_agents,
-                typename AV4<T>::type* xs) {
-  GridParams<T> G = grid_params<T>(a, (const T* const*)x, n, cell_start, cell_agents);
-  const int nb = n > 0 ? (n + kTile - 1) / kTile : 1;
-  k_grid_hist<T, 3><<<nb, kTile, 0, a->stream>>>(G);
-  k_scan_cells<<<a->n_tiles, kTile, 0, a->stream>>>(grid_scan_args(G));
-  k_grid_scatter<T><<<nb, kTile, 0, a->stream>>>(G);
-  k_grid_stable<T><<<nb, kTile, 0, a->stream>>>(G);
-  k_adj_gather<T><<<nb, kTile, 0, a->stream>>>(x[0], x[1], x[2], cell_agents, xs, n);
-}
-
-template <typename T>
 AdjParams<T> adj_params(cbm_adjoint* a, int n) {
   AdjParams<T> A;
   memset(&A, 0, sizeof A);
@@ -390,12 +456,55 @@ AdjParams<T> adj_params(cbm_adjoint* a, int n) {
   A.a = (T)k.k_att;
   A.rho = (T)k.r_rep;
   A.ratt = (T)k.r_att;
-  double c = std::max(k.r_rep, k.r_att), v = c * c * (1.0 + 1e-5);
-  T t = (T)v;
-  A.cut2 = (double)t < v ? std::nextafter(t, (T)INFINITY) : t;
+  const double c = std::max(k.r_rep, k.r_att), up = c * c * (1.0 + 1e-5);
+  const T t = (T)up;
+  A.cut2 = (double)t < up ? std::nextafter(t, (T)INFINITY) : t;
+  auto mid = [](double v) { return v == 0.0 || (std::fabs(v) > 1e-12 && std::fabs(v) < 1e12); };
+  A.mid = mid(k.k_rep) && mid(k.k_att) && c < 1e5;
   A.cap = a->cap;
   A.ctr = a->ctr;
+  A.cell_count = a->cell_count;
+  A.agent_cell = a->agent_cell;
+  A.agent_rank = a->agent_rank;
+  A.cell_tmp = a->cell_tmp;
+  A.cell_of_slot = a->cell_of_slot;
   return A;
+}
+
+// The grid of A.x (already filed in its cells) into A.xs, and the Euler step
+// from there to A.xn.  Every kernel follows a kernel on the stream.
+template <typename T>
+void enqueue_step(cbm_adjoint* a, const AdjParams<T>& A, int* starts, int blocks) {
+  ScanArgs S;
+  S.count = a->cell_count;
+  S.start = starts;
+  S.state = a->scan_state;
+  S.n = a->n_cells;
+  S.n_tiles = a->n_tiles;
+  S.ctr = a->ctr;
+  S.due = nullptr;
+  launch_serial(a->stream, true, k_scan_cells, dim3(a->n_tiles), dim3(kTile), 0, S);
+  launch_serial(a->stream, true, k_adj_scatter<T>, dim3(blocks), dim3(kTile), 0, A);
+  launch_serial(a->stream, true, k_adj_place<T>, dim3(blocks), dim3(kTile), 0, A);
+  Params<T> P;
+  memset(&P, 0, sizeof P);
+  P.PA = A.xs;
+  P.cell_of_slot = A.cell_of_slot;
+  P.cell_start = starts;
+  for (int d = 0; d < 3; ++d) {
+    P.n_cells_d[d] = A.nc[d];
+    P.box_lo[d] = A.lo[d];
+    P.box_hi[d] = A.hi[d];
+  }
+  P.edge = A.edge;
+  P.cut2 = A.cut2;
+  P.k_rep = A.k;
+  P.r_rep = A.rho;
+  P.k_att = A.a;
+  P.r_att = A.ratt;
+  P.att_form = CBM_ATT_FROM_REP;
+  launch_serial(a->stream, true, k_adj_step<T>, dim3((A.n + 31) / 32 + (A.n == 0)), dim3(32), 0, P,
+                A);
 }
 
 // Buffers of a shape and the enqueue of its device work (captured once).
@@ -403,10 +512,11 @@ template <typename T>
 int make_plan(cbm_adjoint* a, Plan& P, int n, int nsteps, int K, bool backward) {
   using V4 = typename AV4<T>::type;
   P.release();
-  const size_t S = sizeof(T), nb = (size_t)std::max(n, 1) * S, n1 = (size_t)std::max(n, 1);
+  const size_t S = sizeof(T), n1 = (size_t)std::max(n, 1), nb = n1 * S, nv = n1 * sizeof(V4);
   const int blocks = n > 0 ? (n + kTile - 1) / kTile : 1;
+  const int step_blocks = n > 0 ? (n + kSlots - 1) / kSlots : 1;
   const int nseg = backward ? std::max((nsteps + K - 1) / K, 1) : 0;
-  const int Kb = backward ? K : 1;
+  const size_t Kb = backward ? (size_t)K : 1;  // steps kept at once
   bool ok = true;
   auto get = [&](size_t bytes) -> void* {
     void* p = nullptr;
@@ -417,31 +527,26 @@ int make_plan(cbm_adjoint* a, Plan& P, int n, int nsteps, int K, bool backward) 
     P.bufs.push_back(p);
     return p;
   };
-  T* fw[2][3];
-  T* ckpt[3] = {};
-  T* seg[3] = {};
-  T* lam[2][3] = {};
   T* tgt[3] = {};
+  V4* lam[2] = {};
   for (int d = 0; d < 3; ++d) {
     P.in_x[d] = get(nb);
-    fw[0][d] = (T*)get(nb);
-    fw[1][d] = (T*)get(nb);
+    P.out_xT[d] = get(nb);
     if (backward) {
       tgt[d] = (T*)get(nb);
       P.in_tgt[d] = tgt[d];
-      ckpt[d] = (T*)get(nb * (size_t)nseg);
-      seg[d] = (T*)get(nb * (size_t)(K + 1));
-      lam[0][d] = (T*)get(nb);
-      lam[1][d] = (T*)get(nb);
+      P.out_dx0[d] = get(nb);
     }
   }
-  int* starts = (int*)get((size_t)(a->n_cells + 1) * 4 * (size_t)Kb);
-  int* agents = (int*)get(n1 * 4 * (size_t)Kb);
-  V4* xs = (V4*)get(n1 * sizeof(V4) * (size_t)Kb);
-  V4* ls = backward ? (V4*)get(n1 * sizeof(V4)) : nullptr;
-  int* pair_n = backward ? (int*)get(n1 * 4 * (size_t)K) : nullptr;
-  int* pair_list = backward ? (int*)get(n1 * 4 * (size_t)a->cap * (size_t)K) : nullptr;
-  P.gpart = (double*)get((size_t)blocks * 3 * 8);
+  V4* fw[2] = {(V4*)get(nv), (V4*)get(nv)};
+  V4* ckpt = backward ? (V4*)get(nv * (size_t)nseg) : nullptr;
+  if (backward)
+    for (int q = 0; q < 2; ++q) lam[q] = (V4*)get(nv);
+  int* starts = (int*)get((size_t)(a->n_cells + 1) * 4);
+  V4* xs = (V4*)get(nv * Kb);
+  int* pair_n = backward ? (int*)get(n1 * 4 * Kb) : nullptr;
+  int* pair_list = (int*)get(n1 * 4 * (size_t)a->cap * Kb);
+  P.gpart = (double*)get((size_t)step_blocks * 3 * 8);
   P.lpart = (double*)get((size_t)blocks * 8);
   if (!ok) {
     P.release();
@@ -452,72 +557,72 @@ int make_plan(cbm_adjoint* a, Plan& P, int n, int nsteps, int K, bool backward) 
   P.K = K;
   P.backward = backward;
   P.blocks = blocks;
+  P.step_blocks = step_blocks;
   cudaStream_t st = a->stream;
   cudaGraph_t g = nullptr;
-  ACUDA(a, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-  // forward sweep, keeping a checkpoint every K steps
-  for (int d = 0; d < 3; ++d)
-    cudaMemcpyAsync(fw[0][d], P.in_x[d], nb, cudaMemcpyDeviceToDevice, st);
-  for (int s = 0; s < nsteps; ++s) {
-    T* const* cur = fw[s % 2];
-    T* const* nxt = fw[(s + 1) % 2];
-    if (backward && s % K == 0)
-      for (int d = 0; d < 3; ++d)
-        cudaMemcpyAsync(ckpt[d] + (size_t)(s / K) * n, cur[d], nb, cudaMemcpyDeviceToDevice, st);
-    build_grid<T>(a, cur, n, starts, agents, xs);
+  // a step from cur to nxt; kept (slot positions and pairs) in place m of the
+  // segment, or, m < 0, in place 0 without its pair counts
+  auto step = [&](const V4* cur, V4* nxt, int m, bool file) {
     AdjParams<T> A = adj_params<T>(a, n);
+    const size_t at = (size_t)(m < 0 ? 0 : m) * n1;
+    A.x = cur;
+    A.xn = nxt;
+    A.xs = xs + at;
     A.cell_start = starts;
-    A.xs = xs;
-    for (int d = 0; d < 3; ++d) A.xn[d] = nxt[d];
-    k_adj_forward<T, false><<<blocks, kTile, 0, st>>>(A);
+    A.pair_n = m < 0 ? nullptr : pair_n + at;
+    A.pair_list = pair_list + at * (size_t)a->cap;
+    A.file = file;
+    enqueue_step<T>(a, A, starts, blocks);
+  };
+  auto file_state = [&](const V4* x) {
+    AdjParams<T> A = adj_params<T>(a, n);
+    A.x = x;
+    k_adj_file<T><<<blocks, kTile, 0, st>>>(A);
+  };
+  ACUDA(a, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+  // forward sweep, keeping a checkpoint at the start of every segment but the
+  // last, whose steps are kept as they are made
+  k_adj_pack<T><<<blocks, kTile, 0, st>>>((const T*)P.in_x[0], (const T*)P.in_x[1],
+                                          (const T*)P.in_x[2], fw[0], n);
+  const int last0 = (nseg - 1) * K;  // first step of the last segment
+  if (nsteps) file_state(fw[0]);
+  for (int s = 0; s < nsteps; ++s) {
+    const V4* cur = fw[s % 2];
+    const bool kept = backward && s >= last0;
+    step(cur, fw[(s + 1) % 2], kept ? s - last0 : -1, s + 1 < nsteps);
+    if (backward && !kept && s % K == 0)
+      k_adj_keep<T><<<blocks, kTile, 0, st>>>(cur, ckpt + (size_t)(s / K) * n1, n);
   }
-  for (int d = 0; d < 3; ++d) P.out_xT[d] = fw[nsteps % 2][d];
+  V4* xT = fw[nsteps % 2];
+  k_adj_unpack<T><<<blocks, kTile, 0, st>>>(xT, (T*)P.out_xT[0], (T*)P.out_xT[1], (T*)P.out_xT[2], n);
   if (backward) {
-    T* const* xT = fw[nsteps % 2];
-    k_adj_loss<T><<<blocks, kTile, 0, st>>>(xT[0], xT[1], xT[2], tgt[0], tgt[1], tgt[2], lam[0][0],
-                                            lam[0][1], lam[0][2], n, P.lpart);
-    cudaMemsetAsync(P.gpart, 0, (size_t)blocks * 3 * 8, st);
+    k_adj_loss<T><<<blocks, kTile, 0, st>>>(xT, tgt[0], tgt[1], tgt[2], lam[0], n, P.lpart);
+    cudaMemsetAsync(P.gpart, 0, (size_t)step_blocks * 3 * 8, st);
     int li = 0;  // lam[li] holds lambda_{n+1}
     for (int sg = nseg - 1; sg >= 0; --sg) {
-      const int n0 = sg * K, n1s = std::min(n0 + K, nsteps), len = n1s - n0;
-      for (int d = 0; d < 3; ++d)
-        cudaMemcpyAsync(seg[d], ckpt[d] + (size_t)sg * n, nb, cudaMemcpyDeviceToDevice, st);
-      // recompute the segment, keeping each step's grid, slot positions and pairs
-      for (int m = 0; m < len; ++m) {
-        T* cur[3];
-        T* nxt[3];
-        for (int d = 0; d < 3; ++d) {
-          cur[d] = seg[d] + (size_t)m * n;
-          nxt[d] = seg[d] + (size_t)(m + 1) * n;
-        }
-        int* gs = starts + (size_t)m * (a->n_cells + 1);
-        int* ga = agents + (size_t)m * n;
-        V4* gx = xs + (size_t)m * n;
-        build_grid<T>(a, cur, n, gs, ga, gx);
-        AdjParams<T> A = adj_params<T>(a, n);
-        A.cell_start = gs;
-        A.xs = gx;
-        A.pair_n = pair_n + (size_t)m * n;
-        A.pair_list = pair_list + (size_t)m * n * a->cap;
-        for (int d = 0; d < 3; ++d) A.xn[d] = nxt[d];
-        k_adj_forward<T, true><<<blocks, kTile, 0, st>>>(A);
+      const int n0 = sg * K, len = std::min(n0 + K, nsteps) - n0;
+      if (sg != nseg - 1) {  // recompute the segment, keeping its steps
+        cudaMemcpyAsync(fw[0], ckpt + (size_t)sg * n1, nv, cudaMemcpyDeviceToDevice, st);
+        file_state(fw[0]);
+        for (int m = 0; m < len; ++m) step(fw[m % 2], fw[(m + 1) % 2], m, m + 1 < len);
       }
       for (int m = len - 1; m >= 0; --m) {
-        int* ga = agents + (size_t)m * n;
-        const int nbk = n > 0 ? (n + kTile - 1) / kTile : 1;
-        k_adj_gather<T><<<nbk, kTile, 0, st>>>(lam[li][0], lam[li][1], lam[li][2], ga, ls, n);
         AdjParams<T> A = adj_params<T>(a, n);
-        A.xs = xs + (size_t)m * n;
-        A.ls = ls;
-        A.pair_n = pair_n + (size_t)m * n;
-        A.pair_list = pair_list + (size_t)m * n * a->cap;
+        const size_t at = (size_t)m * n1;
+        A.xs = xs + at;
+        A.lam = lam[li];
+        A.lam_out = lam[li ^ 1];
+        A.pair_n = pair_n + at;
+        A.pair_list = pair_list + at * (size_t)a->cap;
         A.gpart = P.gpart;
-        for (int d = 0; d < 3; ++d) A.lam_out[d] = lam[li ^ 1][d];
-        k_adj_backward<T><<<blocks, kTile, 0, st>>>(A);
+        // (the first after the memset is a plain launch)
+        launch_serial(st, sg != nseg - 1 || m != len - 1, k_adj_backward<T>, dim3(step_blocks),
+                      dim3(kTile), 0, A);
         li ^= 1;
       }
     }
-    for (int d = 0; d < 3; ++d) P.out_dx0[d] = lam[li][d];
+    k_adj_unpack<T><<<blocks, kTile, 0, st>>>(lam[li], (T*)P.out_dx0[0], (T*)P.out_dx0[1],
+                                              (T*)P.out_dx0[2], n);
   }
   cudaError_t e = cudaStreamEndCapture(st, &g);
   if (e != cudaSuccess) {
@@ -555,7 +660,7 @@ int run(cbm_adjoint* a, const void* const* x0h, int n, int nsteps, int K, const 
       if (xTh[d] && nb) ACUDA(a, cudaMemcpyAsync(xTh[d], P.out_xT[d], nb, cudaMemcpyDeviceToHost, st));
   std::vector<double> gp, lp;
   if (backward) {
-    gp.resize((size_t)P.blocks * 3);
+    gp.resize((size_t)P.step_blocks * 3);
     lp.resize((size_t)P.blocks);
     ACUDA(a, cudaMemcpyAsync(gp.data(), P.gpart, gp.size() * 8, cudaMemcpyDeviceToHost, st));
     ACUDA(a, cudaMemcpyAsync(lp.data(), P.lpart, lp.size() * 8, cudaMemcpyDeviceToHost, st));
@@ -576,10 +681,9 @@ int run(cbm_adjoint* a, const void* const* x0h, int n, int nsteps, int K, const 
   }
   if (backward) {
     double l = 0.0, g[3] = {0.0, 0.0, 0.0};
-    for (int b = 0; b < P.blocks; ++b) {  // fixed order: deterministic
-      l += lp[(size_t)b];
+    for (int b = 0; b < P.blocks; ++b) l += lp[(size_t)b];  // fixed order: deterministic
+    for (int b = 0; b < P.step_blocks; ++b)
       for (int m = 0; m < 3; ++m) g[m] += gp[(size_t)b * 3 + m];
-    }
     if (loss) *loss = n > 0 ? l / (3.0 * (double)n) : 0.0;
     if (dtheta)
       for (int m = 0; m < 3; ++m) dtheta[m] = g[m];
@@ -631,6 +735,10 @@ int cbm_adjoint_create(cbm_adjoint** out, const cbm_config* cfg) {
   a->n_cells = (int)nc;
   a->n_tiles = (a->n_cells + kScanTile - 1) / kScanTile;
   a->cap = std::max(k.n_max_neighbors, 64);
+  if (a->ts == 8)
+    cudaFuncSetAttribute(k_adj_step<double>, cudaFuncAttributePreferredSharedMemoryCarveout, 72);
+  else
+    cudaFuncSetAttribute(k_adj_step<float>, cudaFuncAttributePreferredSharedMemoryCarveout, 72);
   const size_t n = (size_t)std::max(a->n_max, 1);
   bool ok = true;
   auto get = [&](size_t bytes) -> void* {
@@ -647,6 +755,7 @@ int cbm_adjoint_create(cbm_adjoint** out, const cbm_config* cfg) {
   a->agent_cell = (int*)get(n * 4);
   a->agent_rank = (int*)get(n * 4);
   a->cell_tmp = (int*)get(n * 4);
+  a->cell_of_slot = (int*)get(n * 4);
   a->ctr = (Counters*)get(sizeof(Counters));
   if (!ok) {
     for (void* p : a->allocs) cudaFree(p);

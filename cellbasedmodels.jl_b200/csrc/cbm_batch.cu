@@ -328,7 +328,7 @@ __device__ __forceinline__ void list_row_group(const BatchParams& B, const Comm&
 // where it applies, else one by one.
 __device__ __forceinline__ void terms4(const Comm& C, const PairLine<float>& L, const float* xi,
                                        const float4* v, const bool* none, float* acc) {
-  if (L.mid && pair_terms4_mid<true>(L, xi, v, none, acc)) return;
+  if (L.mid && pair_terms4_mid<true>(L, xi, v, none, acc) >= 0) return;
 #pragma unroll
   for (int u = 0; u < 4; ++u)
     if (!none[u]) {

@@ -1227,18 +1227,19 @@ __device__ __forceinline__ PairCoef<T> pair_coef(const Params<T>& P) {
 }
 
 // Soft-sphere pair term (repulsion inside r_rep, attraction up to r_att) of
-// the difference e with squared norm s2, added to acc.
+// the difference e with squared norm s2, added to acc; whether there is one.
 template <typename T, int D>
-__device__ __forceinline__ void pair_term(const PairCoef<T>& c, const T* e, T s2, T* acc) {
-  if (s2 >= c.cut2) return;  // d >= cutoff for certain (NaN takes the exact test)
+__device__ __forceinline__ bool pair_term(const PairCoef<T>& c, const T* e, T s2, T* acc) {
+  if (s2 >= c.cut2) return false;  // d >= cutoff for certain (NaN takes the exact test)
   const T dd = sqrt(s2);
   T F;
   if (dd < c.rrep) F = c.krep * (c.rrep - dd);
   else if (dd < c.ratt) F = c.from_rep ? -(c.katt * (dd - c.rrep)) : -(c.katt * (c.ratt - dd));
-  else return;
+  else return false;
   const T sc = F / dd;
 #pragma unroll
   for (int d = 0; d < D; ++d) acc[d] = acc[d] + sc * e[d];
+  return true;
 }
 
 // Terms of the first nblk stored partner blocks of slot s, oldest first.

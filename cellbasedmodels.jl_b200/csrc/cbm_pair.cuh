@@ -65,12 +65,13 @@ __device__ __forceinline__ PairLine<T> make_pair_line(T cut2, T k_rep, T r_rep, 
 }
 
 // The terms of four partners at positions v, added to acc in order; an entry
-// with none[u] adds nothing.  False, with acc as it was, for distances that
-// need the general square root and quotient (coincident agents; with kFar
-// also infinities, NaN and distances above 1e6).  L.mid must hold.  Square
-// root and quotient are sqrt_mid and div_mid on pairs of values.
+// with none[u] adds nothing.  Returns the entries that lie within the cutoff
+// (bit u), or -1, with acc as it was, for distances that need the general
+// square root and quotient (coincident agents; with kFar also infinities, NaN
+// and distances above 1e6).  L.mid must hold.  Square root and quotient are
+// sqrt_mid and div_mid on pairs of values.
 template <bool kFar>
-__device__ __forceinline__ bool pair_terms4_mid(const PairLine<float>& L, const float* xi,
+__device__ __forceinline__ int pair_terms4_mid(const PairLine<float>& L, const float* xi,
                                                 const float4* v, const bool* none, float* acc) {
   const float2 ixy = make_float2(xi[0], xi[1]);
   float2 exy[4], n2[2];
@@ -83,9 +84,10 @@ __device__ __forceinline__ bool pair_terms4_mid(const PairLine<float>& L, const 
     const float n = (-q.x - q.y) - ez[u] * ez[u];
     (u & 1 ? n2[u >> 1].y : n2[u >> 1].x) = none[u] ? L.nfar2 : n;
   }
-  if (!(fmaxf(fmaxf(n2[0].x, n2[0].y), fmaxf(n2[1].x, n2[1].y)) < -1e-12f)) return false;
+  if (!(fmaxf(fmaxf(n2[0].x, n2[0].y), fmaxf(n2[1].x, n2[1].y)) < -1e-12f)) return -1;
   // (a NaN fails the sum's test, and none's own difference is not looked at)
-  if (kFar && !((n2[0].x + n2[0].y) + (n2[1].x + n2[1].y) > -1e12f)) return false;
+  if (kFar && !((n2[0].x + n2[0].y) + (n2[1].x + n2[1].y) > -1e12f)) return -1;
+  int in = 0;
 #pragma unroll
   for (int p = 0; p < 2; ++p) {
     const float2 x = n2[p], half = make_float2(0.5f, 0.5f);
@@ -106,7 +108,9 @@ __device__ __forceinline__ bool pair_terms4_mid(const PairLine<float>& L, const 
     y = f2_fma(y, f2_fma(d, y, make_float2(1.f, 1.f)), y);
     float2 q = f2_mul(F, y);
     q = f2_fma(f2_fma(d, q, F), y, q);
-    const float c0 = d.x > L.nreach ? q.x : 0.f, c1 = d.y > L.nreach ? q.y : 0.f;
+    const bool i0 = d.x > L.nreach, i1 = d.y > L.nreach;
+    in |= (i0 ? 1 << 2 * p : 0) | (i1 ? 2 << 2 * p : 0);
+    const float c0 = i0 ? q.x : 0.f, c1 = i1 ? q.y : 0.f;
     const float2 t0 = f2_mul(make_float2(c0, c0), exy[2 * p]);
     const float2 t1 = f2_mul(make_float2(c1, c1), exy[2 * p + 1]);
     // scalar sums: a packed product and a packed sum came out fused
@@ -114,7 +118,7 @@ __device__ __forceinline__ bool pair_terms4_mid(const PairLine<float>& L, const 
     acc[1] = (acc[1] + t0.y) + t1.y;
     acc[2] = (acc[2] + c0 * ez[2 * p]) + c1 * ez[2 * p + 1];
   }
-  return true;
+  return in;
 }
 
 }  // namespace cbm

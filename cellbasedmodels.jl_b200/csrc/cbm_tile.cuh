@@ -45,8 +45,18 @@ constexpr float kTileReach = 100.f;
 // largest half)
 constexpr double kTileMaxCutoff = 50.0;
 
+template <typename S>
+__device__ __forceinline__ void tile_begin(S& s) {  // the empty word
+  s.word[kTileWords * 32 + (threadIdx.x & 31)] = 0u;
+  s.base[kTileWords] = 0;
+}
+
+// Near candidates a lane holds when it walks its own; its runs lie above them.
+constexpr int kNearQueue = 24;
+static_assert(kNearQueue * 32 + 2 * 9 * 32 <= kTileWords * 32, "queue and runs fit the words");
 struct TileSmem {
-  unsigned word[(kTileWords + 1) * 32];  // decisions of word w, agent a; then an empty word
+  // decisions of word w, agent a; then an empty word
+  alignas(8) unsigned word[(kTileWords + 1) * 32];
   int base[kTileWords + 1];              // first slot of word w
   unsigned short info[kTileWords];       // run (0..8) | number of candidates << 8
   __align__(16) unsigned char rec[4 * kTileWordStride];  // records of four words
@@ -134,14 +144,18 @@ __device__ __forceinline__ PairLine<T> pair_line(const Params<T>& P) {
 
 // The terms of four partners at positions v, added to acc in order; an entry
 // that is the agent itself adds nothing.  `plain`: the positions are within
-// kTileReach of one another and L.mid holds.
+// kTileReach of one another and L.mid holds.  Returns the entries within the
+// cutoff (bit u).
 template <typename T>
-__device__ __forceinline__ void pair_terms4(const PairCoef<T>& c, const PairLine<T>& L, bool plain,
+__device__ __forceinline__ int pair_terms4(const PairCoef<T>& c, const PairLine<T>& L, bool plain,
                                             const T* xi, const typename V4T<T>::type* v, int s,
                                             const int* qq, T* acc) {
   if constexpr (std::is_same<T, float>::value) {
     const bool none[4] = {qq[0] == s, qq[1] == s, qq[2] == s, qq[3] == s};
-    if (plain && pair_terms4_mid<false>(L, xi, v, none, acc)) return;
+    if (plain) {
+      const int in = pair_terms4_mid<false>(L, xi, v, none, acc);
+      if (in >= 0) return in;
+    }
   }
   if constexpr (std::is_same<T, double>::value) {
     double e[4][3], n2[4];
@@ -154,6 +168,7 @@ __device__ __forceinline__ void pair_terms4(const PairCoef<T>& c, const PairLine
     }
     if (plain && fmin(fmin(n2[0], n2[1]), fmin(n2[2], n2[3])) > 1e-12) {
       double sc[4];
+      int in = 0;
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         double y;
@@ -162,29 +177,33 @@ __device__ __forceinline__ void pair_terms4(const PairCoef<T>& c, const PairLine
         const double F = (rep ? L.krep : L.katt) * ((rep ? L.rrep : L.abase) - d);
         const double q = div_mid(F, d, y);
         sc[u] = d < -L.nreach ? q : 0.0;
+        in |= d < -L.nreach ? 1 << u : 0;
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u)
 #pragma unroll
         for (int k = 0; k < 3; ++k) acc[k] = acc[k] + sc[u] * e[u][k];
-      return;
+      return in;
     }
   }
+  int in = 0;
 #pragma unroll
   for (int u = 0; u < 4; ++u)
     if (qq[u] != s) {
       T xj[3], e[3];
       to3<T>(v[u], xj);
       const T d2 = pair_diff<T, 3>(xi, xj, e);
-      pair_term<T, 3>(c, e, d2, acc);
+      if (pair_term<T, 3>(c, e, d2, acc)) in |= 1 << u;
     }
+  return in;
 }
 
 // The pair forces of the 32 slots from s0 on (lanes beyond N idle), summed
-// into acc in the reference's order.
-template <typename T>
+// into acc in the reference's order; partner(slot) is told of every pair with
+// a force, in that order.
+template <typename T, typename F>
 __device__ __forceinline__ void tile_forces(const Params<T>& P, TileSmem& S, const int N,
-                                            const int s0, const T* xi, T* acc) {
+                                            const int s0, const T* xi, T* acc, F&& partner) {
   using V4 = typename V4T<T>::type;
   const int lane = threadIdx.x & 31;
   const bool in = s0 + lane < N;
@@ -236,39 +255,87 @@ __device__ __forceinline__ void tile_forces(const Params<T>& P, TileSmem& S, con
     return words;
   };
   // A word costs the warp about 75 instructions, a row of agents about 350,
-  // and a candidate tested by each lane about 14: sparse tiles, whose agents
-  // lie in many cells with a few candidates each, test their own.
+  // and a candidate tested by each lane about 20: sparse tiles, whose agents
+  // lie in many cells with a few candidates each, test their own.  (All tiles
+  // by words against all by lanes: the young colony's kernel 46 us against
+  // 76, the 256^3 medium's 159 against 55, the adjoint's 65536 agents at 0.13
+  // per unit volume 195 against 115 us a step.)
   const int most = __reduce_max_sync(kFull, in ? cand : 0);
-  bool by_tile = 14 * most > 350 * n_rows;
+  bool by_tile = 20 * most > 350 * n_rows && P.cut2 <= (T)(1.1 * kTileMaxCutoff * kTileMaxCutoff);
   if (by_tile) {
     int words = 0;
     for (unsigned l = leaders; l; l &= l - 1u)
       words += unite(__shfl_sync(kFull, peers, __ffs(l) - 1));
-    by_tile = 75 * words + 350 * n_rows < 14 * most;
+    by_tile = 75 * words + 350 * n_rows < 20 * most;
   }
   const PairLine<T> line = pair_line(P);
   if (!by_tile) {
-    if (!in) return;
+    // Each lane walks its own candidates, four at a time, passing over empty
+    // runs (most of a sparse tile's are), the next four's positions in flight; those that may be near wait in the lane's column of
+    // S.word and are evaluated together.  Runs as first slot and end, by lane.
+    int2* const runs = reinterpret_cast<int2*>(S.word + 32 * kNearQueue);
 #pragma unroll
-    for (int r = 0; r < 9; ++r)
-      for (int q = lo[r]; q < hi[r]; q += 4) {  // beyond the run: the agent itself
+    for (int r = 0; r < 9; ++r) runs[r * 32 + lane] = make_int2(lo[r], hi[r]);
+    int r = 0, q = lo[0], e = in ? hi[0] : lo[0], nq = 0;
+    if (!in) r = 8;
+    auto take = [&](int* qq, V4* v) {
+      while (q >= e && r < 8) {
+        const int2 run = runs[++r * 32 + lane];
+        q = run.x;
+        e = run.y;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) qq[u] = q + u < e ? q + u : s;
+      q += 4;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = U[qq[u]];
+    };
+    auto evaluate = [&]() {
+      for (int k = 0; __any_sync(kFull, k < nq); k += 4) {
         int qq[4];
         V4 v[4];
-        bool near = false, plain = line.mid;
+        bool plain = line.mid;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) qq[u] = q + u < hi[r] ? q + u : s;
+        for (int u = 0; u < 4; ++u) qq[u] = k + u < nq ? (int)S.word[(k + u) * 32 + lane] : s;
 #pragma unroll
         for (int u = 0; u < 4; ++u) v[u] = U[qq[u]];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          T xj[3], e[3];
+          T xj[3], d[3];
           to3<T>(v[u], xj);
-          const T d2 = pair_diff<T, 3>(xi, xj, e);
-          near = near || (qq[u] != s && !(d2 >= coef.cut2));
-          plain = plain && d2 < (T)1e12;
+          plain = plain && pair_diff<T, 3>(xi, xj, d) < (T)1e12;
         }
-        if (near) pair_terms4<T>(coef, line, plain, xi, v, s, qq, acc);
+        const int hit = pair_terms4<T>(coef, line, plain, xi, v, s, qq, acc);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if ((hit >> u) & 1) partner(qq[u]);
       }
+      nq = 0;
+    };
+    int qq[4];
+    V4 v[4];
+    take(qq, v);
+    while (true) {
+      const bool more = __any_sync(kFull, q < e || r < 8);
+      int qn[4];
+      V4 vn[4];
+      if (more) take(qn, vn);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        T xj[3], d[3];
+        to3<T>(v[u], xj);
+        S.word[nq * 32 + lane] = (unsigned)qq[u];  // kept when it may be near (or is NaN)
+        nq += qq[u] != s && !(pair_diff<T, 3>(xi, xj, d) >= coef.cut2) ? 1 : 0;
+      }
+      if (!more || __any_sync(kFull, nq > kNearQueue - 5)) evaluate();
+      if (!more) break;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        qq[u] = qn[u];
+        v[u] = vn[u];
+      }
+    }
+    __syncwarp();
     return;
   }
 
@@ -450,7 +517,10 @@ __device__ __forceinline__ void tile_forces(const Params<T>& P, TileSmem& S, con
       V4 v[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) v[u] = U[qq[u]];
-      pair_terms4<T>(coef, line, plain, xi, v, s, qq, acc);
+      const int hit = pair_terms4<T>(coef, line, plain, xi, v, s, qq, acc);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if ((hit >> u) & 1) partner(qq[u]);
     }
     if (last) return;
     free_to += kTileRefill;
@@ -470,14 +540,13 @@ __global__ void __launch_bounds__(32, kTileWarps) k_agent_de_tile(Params<T> P) {
   const int N = (int)C->N[P.parity];
   const int n_tiles = (N + 31) >> 5;
   const int lane = threadIdx.x & 31;
-  S.word[kTileWords * 32 + lane] = 0u;
-  S.base[kTileWords] = 0;
+  tile_begin(S);
   int tile = (int)blockIdx.x;
   while (tile < n_tiles) {
     const int s = tile * 32 + lane;
     T xi[3], acc[3] = {(T)0, (T)0, (T)0};
     to3<T>(P.PA[s < N ? s : N - 1], xi);
-    tile_forces<T>(P, S, N, tile * 32, xi, acc);
+    tile_forces<T>(P, S, N, tile * 32, xi, acc, [](int) {});
     if (s < N) finish_agent<T, 3>(P, s, xi, acc);
     __syncwarp();
     int t = 0;
