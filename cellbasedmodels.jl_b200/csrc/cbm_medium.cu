@@ -31,6 +31,9 @@
 #include <vector>
 
 #include "../../include/cbm_b200.h"
+#include "cbm_common.cuh"
+
+using namespace cbm;
 
 namespace {
 
@@ -101,36 +104,81 @@ __device__ __forceinline__ void cp_async_wait_all() {
 }
 
 // One line's solve in place: X(j) is node j of the line (ends 0 and n-1).
-// The table entries and nodes of the next iteration are loaded one step
-// ahead, so that only the arithmetic stays on the recurrence's chain.
+// Table entries and nodes are read in groups of kAhead, the next group before
+// the current one's arithmetic, so that only the arithmetic stays on the
+// recurrence's chain (57 cycles a node forwards in Float32, two conversions
+// and a Float64 product among them, and 23 backwards; read one node ahead it
+// was about 300 in all).
+constexpr int kAhead = 4;
 template <typename T, typename F>
 __device__ __forceinline__ void line_solve(F&& X, int n, T sub, T main, T sup, const T* cs,
                                            const double* pv) {
   T d = (X(1) - sub * X(0)) / main;
   X(1) = d;
-  double pn = pv[2];
-  T xn = X(2);
-  for (int j = 2; j <= n - 3; ++j) {
-    const double p = pn;
-    const T xj = xn;
-    pn = pv[j + 1];
-    xn = X(j + 1);
-    d = (T)((double)(xj - sub * d) * p);
-    X(j) = d;
-  }
-  T x = (T)((double)((xn - sup * X(n - 1)) - sub * d) * pn);
-  X(n - 2) = x;
-  T cn = n - 3 >= 1 ? cs[n - 3] : (T)0;
-  T dn = n - 3 >= 1 ? X(n - 3) : (T)0;
-  for (int j = n - 3; j >= 1; --j) {
-    const T c = cn, dj = dn;
-    if (j > 1) {
-      cn = cs[j - 1];
-      dn = X(j - 1);
+  const T end = X(n - 1);
+  double p[kAhead], pq[kAhead];
+  T x[kAhead], xq[kAhead];
+  auto forward = [&](int j, double* pp, T* xx) {  // nodes j .. j + 3, up to n - 2
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int k = j + u < n - 2 ? j + u : n - 2;
+      pp[u] = pv[k];
+      xx[u] = X(k);
     }
-    x = dj - c * x;
-    X(j) = x;
+  };
+  forward(2, p, x);
+  int j = 2;
+  for (; j + kAhead <= n - 2; j += kAhead) {  // nodes below n - 2
+    forward(j + kAhead, pq, xq);
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      d = (T)((double)(x[u] - sub * d) * p[u]);
+      X(j + u) = d;
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      p[u] = pq[u];
+      x[u] = xq[u];
+    }
   }
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u)
+    if (j + u < n - 2) {
+      d = (T)((double)(x[u] - sub * d) * p[u]);
+      X(j + u) = d;
+    }
+  d = (T)((double)((X(n - 2) - sup * end) - sub * d) * pv[n - 2]);
+  X(n - 2) = d;
+  T c[kAhead], cq[kAhead];
+  auto backward = [&](int k, T* cc, T* dd) {  // nodes k .. k - 3, down to 1
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int q = k - u > 1 ? k - u : 1;
+      cc[u] = cs[q];
+      dd[u] = X(q);
+    }
+  };
+  j = n - 3;
+  if (j >= 1) backward(j, c, x);
+  for (; j - kAhead >= 0; j -= kAhead) {
+    backward(j - kAhead, cq, xq);
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      d = x[u] - c[u] * d;
+      X(j - u) = d;
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      c[u] = cq[u];
+      x[u] = xq[u];
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u)
+    if (j - u >= 1) {
+      d = x[u] - c[u] * d;
+      X(j - u) = d;
+    }
 }
 
 // The Thomas solves of axis A: one thread per (field, line through interior
@@ -174,23 +222,26 @@ __global__ void __launch_bounds__(kSweepThreads)
   line_solve<T>([&](int j) -> T& { return Y[j * st]; }, n, sub, main, sup, cs, pv);
 }
 
-// The same solves with the lines of one warp staged in shared memory: 32
-// lines per block, copied in and out with coalesced accesses (rows along x
-// for axis 0; for axes 1 and 2, 32 consecutive lines at each position along
-// them) and solved in place there.  Row r of the tile is line r of the block:
-// at r * rowp + j for axis 0 (rowp odd, so the 32 rows fall in distinct
-// banks), at j * 32 + r otherwise.
+// The same solves with 32 lines staged in shared memory: four warps copy them
+// in and out with coalesced accesses (rows along x for axis 0, with the
+// explicit part on the way in; for axes 1 and 2, 32 consecutive lines at each
+// position along them), one warp solves them in place.  A solve is one serial
+// recurrence a line, whose latency nothing hides (101^3 nodes and two fields
+// are 613 such warps, one a scheduler), so what surrounds it is made short:
+// with one warp a block for everything the three sweeps of a step took 27, 18
+// and 18 us.  Row r of the tile is line r of the block: at r * rowp + j for
+// axis 0 (rowp odd, so the 32 rows fall in distinct banks), at j * 32 + r
+// otherwise.
 constexpr int kTileLines = 32;
+constexpr int kTileWarps = 4;
 
 template <typename T, int A, int D>
-__global__ void __launch_bounds__(kTileLines)
+__global__ void __launch_bounds__(kTileLines * kTileWarps)
     k_dgadi_sweep_tiled(const T* __restrict__ xo, T* __restrict__ xn,
                         const FieldCoef<T>* __restrict__ coef, const T* __restrict__ cstar,
                         const double* __restrict__ piv, int nmax, int n0, int n1, int n2, int nf,
                         int rowp, const T* __restrict__ src, T cmax) {
   extern __shared__ __align__(16) unsigned char med_smem[];
-  T* tile = reinterpret_cast<T*>(med_smem);
-  T* stile = tile + kTileLines * rowp;  // axis 0: the source rows
   const int len[3] = {n0, n1, n2};
   const long long stride[3] = {1, n0, (long long)n0 * n1};
   constexpr int B = A == 0 ? 1 : 0;
@@ -199,57 +250,79 @@ __global__ void __launch_bounds__(kTileLines)
   const long long lines = (long long)nb * nc;
   const int n = len[A];
   const long long st = stride[A];
-  const int t = threadIdx.x;
-  // global offset of the first node of line (block base + r), or -1 past the end
-  auto line_base = [&](int r, int* field) -> long long {
-    const long long id = (long long)blockIdx.x * kTileLines + r;
-    if (id >= lines * nf) return -1;
-    const int f = (int)(id / lines);
+  const int t = threadIdx.x & 31, w = threadIdx.x >> 5;
+  // the tables of the block's first line's field and of the one after it
+  // (later ones, where a field has fewer than 32 lines, are read in place),
+  // then the tile
+  double* const tp = reinterpret_cast<double*>(med_smem);
+  T* const tc = reinterpret_cast<T*>(tp + 2 * n);
+  T* const tile = tc + 2 * n;
+  const int f0 = (int)((long long)blockIdx.x * kTileLines / lines);
+  for (int k = threadIdx.x; k < 2 * n; k += kTileLines * kTileWarps) {
+    const int ff = f0 + (k >= n), j = k >= n ? k - n : k;
+    if (ff < nf && j >= 1) {
+      const size_t q = (size_t)(ff * 3 + A) * nmax + j;
+      if (j >= 2 && j < n - 1) tp[k] = piv[q];
+      if (j < n - 2) tc[k] = cstar[q];
+    }
+  }
+  // global offset of the first node of line (block base + t), or -1 past the end
+  int f = 0;
+  long long o = -1;
+  const long long id = (long long)blockIdx.x * kTileLines + t;
+  if (id < lines * nf) {
+    f = (int)(id / lines);
     const long long l = id - (long long)f * lines;
     const int ib = (int)(l % nb) + (B < D ? 1 : 0);
     const int ic = (int)(l / nb) + (Cx < D ? 1 : 0);
-    *field = f;
-    return (long long)f * n0 * n1 * n2 + (long long)ib * stride[B] + (long long)ic * stride[Cx];
-  };
-  int f = 0;
-  const long long o = line_base(t, &f);
+    o = (long long)f * n0 * n1 * n2 + (long long)ib * stride[B] + (long long)ic * stride[Cx];
+  }
   auto at = [&](int r, int j) -> T& { return A == 0 ? tile[r * rowp + j] : tile[j * kTileLines + r]; };
   const long long fnodes = (long long)n0 * n1 * n2;
-  if (A == 0) {
-    for (int r = 0; r < kTileLines; ++r) {
+  pdl_wait();
+  if (A == 0) {  // every row's copies are in flight together
+    T* const stile = tile + kTileLines * rowp;
+    for (int r = w; r < kTileLines; r += kTileWarps) {
       const long long orow = __shfl_sync(kFullMask, o, r);
       const int frow = __shfl_sync(kFullMask, f, r);
       if (orow < 0) break;
-      const long long srow = orow - (long long)frow * fnodes;
+      const T* s = src + (orow - (long long)frow * fnodes);
       for (int j = t; j < n; j += kTileLines) {
         cp_async_elem(&at(r, j), xo + orow + j);
-        cp_async_elem(&stile[r * rowp + j], src + srow + j);
+        cp_async_elem(&stile[r * rowp + j], s + j);
       }
     }
-  } else if (o >= 0) {
-    for (int j = 0; j < n; ++j) cp_async_elem(&at(t, j), xo + o + j * st);
-  }
-  cp_async_wait_all();
-  __syncwarp();
-  if (o >= 0) {
-    if (A == 0) {
-      const T dec = coef->decay[f];
-      for (int j = 1; j < n - 1; ++j) at(t, j) = explicit_part(at(t, j), stile[t * rowp + j], cmax, dec);
+    cp_async_wait_all();  // a thread reads back what it copied itself
+    for (int r = w; r < kTileLines; r += kTileWarps) {
+      const int frow = __shfl_sync(kFullMask, f, r);
+      if (__shfl_sync(kFullMask, o, r) < 0) break;
+      const T dec = coef->decay[frow];
+      for (int j = t; j < n; j += kTileLines)
+        if (j > 0 && j < n - 1) at(r, j) = explicit_part(at(r, j), stile[r * rowp + j], cmax, dec);
     }
+  } else if (o >= 0) {
+    for (int j = w; j < n; j += kTileWarps) cp_async_elem(&at(t, j), xo + o + j * st);
+    cp_async_wait_all();
+  }
+  __syncthreads();
+  if (w == 0 && o >= 0) {
     const T sub = coef->sub[f], main = coef->main[f], sup = coef->sup[f];
-    const T* cs = cstar + (size_t)(f * 3 + A) * nmax;
-    const double* pv = piv + (size_t)(f * 3 + A) * nmax;
+    const bool staged = f - f0 < 2;
+    const T* cs = staged ? tc + (f - f0) * n : cstar + (size_t)(f * 3 + A) * nmax;
+    const double* pv = staged ? tp + (f - f0) * n : piv + (size_t)(f * 3 + A) * nmax;
     line_solve<T>([&](int j) -> T& { return at(t, j); }, n, sub, main, sup, cs, pv);
   }
-  __syncwarp();
+  __syncthreads();
   if (A == 0) {
-    for (int r = 0; r < kTileLines; ++r) {
+#pragma unroll 2
+    for (int r = w; r < kTileLines; r += kTileWarps) {
       const long long orow = __shfl_sync(kFullMask, o, r);
       if (orow < 0) break;
       for (int j = 1 + t; j < n - 1; j += kTileLines) xn[orow + j] = at(r, j);
     }
   } else if (o >= 0) {
-    for (int j = 1; j < n - 1; ++j) xn[o + j * st] = at(t, j);
+#pragma unroll 4
+    for (int j = 1 + w; j < n - 1; j += kTileWarps) xn[o + j * st] = at(t, j);
   }
 }
 
@@ -331,9 +404,9 @@ constexpr size_t kFusedMaxBytes = 200 * 1024;
 template <typename T>
 size_t tile_bytes(int axis, int n) {
   const int rowp = axis == 0 ? (n | 1) : n;
-  return (axis == 0 ? 2 : 1) * (size_t)kTileLines * rowp * sizeof(T);
+  return (axis == 0 ? 2 : 1) * (size_t)kTileLines * rowp * sizeof(T) + 2 * (size_t)n * (sizeof(double) + sizeof(T));
 }
-constexpr size_t kTileMaxBytes = 96 * 1024;
+constexpr size_t kTileMaxBytes = 200 * 1024;  // of the 227 KB a block may have
 
 }  // namespace
 
@@ -384,7 +457,7 @@ void mfree(cbm_medium* m) {
 }
 
 template <typename T, int D>
-int enqueue_step(cbm_medium* m) {
+int enqueue_step(cbm_medium* m, bool pdl) {  // pdl: the operation before is a kernel
   const cbm_medium_config& k = m->cfg;
   const int n0 = k.n[0], n1 = D > 1 ? k.n[1] : 1, n2 = D > 2 ? k.n[2] : 1;
   const int nf = k.n_fields;
@@ -407,15 +480,16 @@ int enqueue_step(cbm_medium* m) {
     const size_t tb = tile_bytes<T>(A, len[A]);
     if (tb <= kTileMaxBytes) {
       const long long nl = lines(A);
-      k_dgadi_sweep_tiled<T, A, D>
-          <<<(unsigned)((nl + kTileLines - 1) / kTileLines), kTileLines, tb, m->stream>>>(
-              u[m->cur], u[m->cur ^ 1], coef, cs, m->piv, m->nmax, n0, n1, n2, nf,
-              A == 0 ? (len[A] | 1) : len[A], src, cmax);
+      launch_serial(m->stream, pdl, k_dgadi_sweep_tiled<T, A, D>,
+                    dim3((unsigned)((nl + kTileLines - 1) / kTileLines)),
+                    dim3(kTileLines * kTileWarps), tb, u[m->cur], u[m->cur ^ 1], coef, cs, m->piv,
+                    m->nmax, n0, n1, n2, nf, A == 0 ? (len[A] | 1) : len[A], src, cmax);
     } else {
       k_dgadi_sweep<T, A, D><<<grid(lines(A)), kSweepThreads, 0, m->stream>>>(
           u[m->cur], u[m->cur ^ 1], coef, cs, m->piv, m->nmax, n0, n1, n2, nf, src, cmax);
     }
     m->cur ^= 1;
+    pdl = true;
   };
   sweep(std::integral_constant<int, 0>());
   if constexpr (D > 1) sweep(std::integral_constant<int, 1>());
@@ -468,11 +542,11 @@ bool set_tile_attrs(int dims, int bytes) {
 }
 
 template <typename T>
-int enqueue_step_t(cbm_medium* m) {
+int enqueue_step_t(cbm_medium* m, bool pdl) {
   switch (m->cfg.dims) {
-    case 1: return enqueue_step<T, 1>(m);
-    case 2: return enqueue_step<T, 2>(m);
-    default: return enqueue_step<T, 3>(m);
+    case 1: return enqueue_step<T, 1>(m, pdl);
+    case 2: return enqueue_step<T, 2>(m, pdl);
+    default: return enqueue_step<T, 3>(m, pdl);
   }
 }
 
@@ -592,7 +666,7 @@ int cbm_medium_step(cbm_medium* m, int32_t nsteps, int32_t flags) {
     }
   } else {
     for (int s = 0; s < nsteps; ++s) {
-      const int rc = m->tsize == 8 ? enqueue_step_t<double>(m) : enqueue_step_t<float>(m);
+      const int rc = m->tsize == 8 ? enqueue_step_t<double>(m, s > 0) : enqueue_step_t<float>(m, s > 0);
       if (rc != CBM_OK) return rc;
       m->steps += 1;
       m->t += m->cfg.dt;  // obj.t += dt
