@@ -1430,7 +1430,8 @@ bool small_eligible(const cbm_ctx* c) {
   return k.neighbors == CBM_NEIGH_CELL_LINKED && k.fate == CBM_FATE_NONE && !k.growth &&
          !k.medium && k.force_mode == CBM_FORCE_DIRECT &&
          (k.integrator == CBM_INT_EULER || k.integrator == CBM_INT_EM) &&
-         c->n_cells <= kSmallMaxCells && c->n_loaded > 0 && c->n_loaded <= kSmallMaxAgents;
+         c->n_cells <= kSmallMaxCells && c->n_loaded > 0 &&
+         c->n_loaded <= (c->tsize == 8 ? kSmallMaxAgents<double> : kSmallMaxAgents<float>);
 }
 
 template <typename T, int D>
@@ -1440,15 +1441,19 @@ struct SmallSteps {
     int n_cells = c->n_cells;
     const size_t smem = (size_t)(n_cells + 1) * sizeof(int);
     auto kern = k_small_steps<T, D>;
-    // one cluster: as many blocks as four lanes an agent need, up to 16
-    long long want = (c->n_loaded * kSmallLanes + kSmallThreads - 1) / kSmallThreads;
-    int blocks = (int)std::max<long long>(1, std::min<long long>(want, kSmallMaxBlocks));
+    // one cluster of sixteen blocks, of the threads that four lanes an agent
+    // need (a community of a few agents: of as many blocks as it fills)
+    const long long lanes = c->n_loaded * kSmallLanes;
+    int blocks = (int)std::max<long long>(
+        1, std::min<long long>((lanes + kSmallMinThreads - 1) / kSmallMinThreads, kSmallMaxBlocks));
+    const long long each = ((lanes + blocks - 1) / blocks + 31) / 32 * 32;
+    const int threads = (int)std::max<long long>(kSmallMinThreads, std::min<long long>(each, kSmallMaxThreads));
     *err = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (*err != cudaSuccess) return;
     cudaLaunchConfig_t lc = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    lc.blockDim = dim3(kSmallThreads);
+    lc.blockDim = dim3((unsigned)threads);
     lc.dynamicSmemBytes = smem;
     lc.stream = c->stream;
     lc.attrs = attr;

@@ -158,6 +158,12 @@ __device__ __forceinline__ float div_mid(float a, float b) {
   const float q = a * y;
   return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
 }
+// (the forms of the two types alike, for templates)
+__device__ __forceinline__ float sqrt_mid(float x, float* inv) {
+  *inv = 0.f;
+  return sqrt_mid(x);
+}
+__device__ __forceinline__ float div_mid(float a, float b, float) { return div_mid(a, b); }
 // *inv: 1 / sqrt(x) to about an ulp, from which div_mid starts
 __device__ __forceinline__ double sqrt_mid(double x, double* inv) {
   double y;

@@ -1351,9 +1351,11 @@ __device__ __forceinline__ void hist_begin(const Params<T>& P) {
 // pushing walls, the lagged force, linear drift and chemotaxis, then the
 // integrator (Euler or Euler-Maruyama), the commit of the written slot and
 // the displacement check of the Verlet algorithms.  xi: the positions the
-// step reads (the stage's, the rule's reflected ones, or the committed ones).
+// step reads (the stage's, the rule's reflected ones, or the committed ones);
+// x_new, when given, gets the new position.
 template <typename T, int D>
-__device__ __forceinline__ void finish_agent(const Params<T>& P, const int s, const T* xi, T* acc) {
+__device__ __forceinline__ void finish_agent(const Params<T>& P, const int s, const T* xi, T* acc,
+                                             T* x_new = nullptr) {
   const int p = P.parity;
   if (P.walls == CBM_WALLS_PUSH) {
 #pragma unroll
@@ -1423,6 +1425,10 @@ __device__ __forceinline__ void finish_agent(const Params<T>& P, const int s, co
     for (int d = 0; d < D; ++d) xn[d] = xi[d] + dv[d] * P.dt;
   }
   P.PB[s] = from3<T>(xn);
+  if (x_new) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) x_new[d] = xn[d];
+  }
   if (kHistInDE<D> && P.hist_in_de) {  // no births or deaths, and every step re-sorts
     const int c = cell_of_pos<T, D>(P, xn);
     P.s_cell[s] = c;

@@ -27,9 +27,19 @@
 
 namespace cbm {
 
-constexpr int kSmallThreads = 1024;
+// Threads a block: four lanes an agent over the sixteen blocks, so that a
+// community of fewer than 4096 agents has fewer warps a scheduler instead of
+// fewer blocks (700 agents: 19.2 us a step as three blocks of 1024 threads,
+// 15.7 as eleven of 256).
+constexpr int kSmallMaxThreads = 1024, kSmallMinThreads = 256;
 constexpr int kSmallMaxBlocks = 16;     // blocks of the cluster (16 needs the non-portable size)
-constexpr int kSmallMaxAgents = 32768;  // communities stepped by one launch (fate-free CellLinked)
+// Communities stepped by one launch (fate-free CellLinked).  The step graph
+// takes much the same time whatever their size (27 us in 2D, 44 in 3D in
+// Float64; 24 and 38 in Float32), the cluster's sixteen SMs take theirs in
+// proportion once their lanes are all in use: Float64 19 and 37 us at 4096
+// agents, 28 and 53 at 5500; Float32 20 and 36 at 5500, 28 and 53 at 9000.
+template <typename T>
+constexpr int kSmallMaxAgents = sizeof(T) == 8 ? 4096 : 6144;
 constexpr int kSmallMaxCells = 8192;    // cell grids a block scans in shared memory
 
 // Barrier of the cluster's blocks: every thread arrives with release and
@@ -43,7 +53,8 @@ __device__ __forceinline__ void cluster_barrier() {
 // Exclusive scan of counts[0, n) by one block into out[0, n]; out[n] = total.
 __device__ __forceinline__ void block_scan_counts(const int* counts, int n, int* out,
                                                   int* warp_sums) {
-  const int per = (n + kSmallThreads - 1) / kSmallThreads;
+  const int nth = (int)blockDim.x;
+  const int per = (n + nth - 1) / nth;
   const int c0 = min(n, (int)threadIdx.x * per), c1 = min(n, c0 + per);
   int local = 0;
   for (int c = c0; c < c1; ++c) {
@@ -61,13 +72,13 @@ __device__ __forceinline__ void block_scan_counts(const int* counts, int n, int*
   if (lane == 31) warp_sums[w] = x;
   __syncthreads();
   if (w == 0) {
-    int v = lane < kSmallThreads / 32 ? warp_sums[lane] : 0;
+    int v = lane < nth / 32 ? warp_sums[lane] : 0;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int y = __shfl_up_sync(kFull, v, o);
       if (lane >= o) v += y;
     }
-    if (lane < kSmallThreads / 32) warp_sums[lane] = v;
+    if (lane < nth / 32) warp_sums[lane] = v;
   }
   __syncthreads();
   int run = (w > 0 ? warp_sums[w - 1] : 0) + x - local;
@@ -76,22 +87,28 @@ __device__ __forceinline__ void block_scan_counts(const int* counts, int n, int*
     out[c] = run;
     run += v;
   }
-  if (threadIdx.x == kSmallThreads - 1) out[n] = warp_sums[kSmallThreads / 32 - 1];
+  if ((int)threadIdx.x == nth - 1) out[n] = warp_sums[nth / 32 - 1];
   __syncthreads();
 }
 
 // agentStepDE! of slot s for CellLinked, by the kSmallLanes lanes of a group
-// (lane gl of the group takes candidates gl, gl + kSmallLanes, ... of each
-// run): the candidates of the 3^D cells in the reference's order, the pair
-// terms of each chunk added in candidate order through the group's shuffles,
-// so the sums are those of k_agent_de (skipping cells with no partner, as its
-// pruning does, changes no sum).  With reflecting walls the rule's reflected
-// positions are computed from the committed ones, here for xi and every
-// candidate.  The group's first lane integrates.
+// (lane gl of the group takes candidates gl, gl + kSmallLanes, ... of the
+// three rows of cells of a plane, one sequence): the candidates of the 3^D
+// cells in the reference's order, the pair terms of each chunk added in
+// candidate order through the group's shuffles, so the sums are those of
+// k_agent_de (skipping cells with no partner, as its pruning does, changes no
+// sum, nor does adding the zero of a candidate beyond the cutoff).  A chunk
+// is one serial chain of position load, root, quotient and ordered sums: the
+// next chunk's positions are loaded before it, and root and quotient take the
+// branch-free forms.  With reflecting walls the rule's reflected positions
+// are computed from the committed ones, here for xi and every candidate.
+// `start`: the grid's offsets, in shared memory.  The group's first lane
+// integrates.
 constexpr int kSmallLanes = 4;
 
 template <typename T, int D>
-__device__ __forceinline__ void small_de(const Params<T>& P, int s) {
+__device__ __forceinline__ void small_de(const Params<T>& P, const PairLine<T>& line,
+                                         const int* start, int s, T* x_new) {
   constexpr int L = kSmallLanes;
   const int lane = threadIdx.x & 31, gl = lane & (L - 1);
   const unsigned gmask = ((1u << L) - 1u) << (lane & ~(L - 1));
@@ -109,7 +126,6 @@ __device__ __forceinline__ void small_de(const Params<T>& P, int s) {
   T xi[3] = {(T)0, (T)0, (T)0};
   pos(s, xi);
   T acc[3] = {(T)0, (T)0, (T)0};
-  const PairCoef<T> coef = pair_coef<T>(P);
   int q3[3] = {0, 0, 0};
   cell_coords<D>(P.n_cells_d, cell_of_pos<T, D>(P, xi), q3);
   const int nx = P.n_cells_d[0];
@@ -118,52 +134,55 @@ __device__ __forceinline__ void small_de(const Params<T>& P, int s) {
   for (int dz = 0; dz < nz_rows; ++dz) {
     const int pz = D > 2 ? q3[2] + dz - 1 : 0;
     if (D > 2 && (pz < 0 || pz >= P.n_cells_d[2])) continue;
-    for (int dy = 0; dy < ny_rows; ++dy) {
-      const int py = D > 1 ? q3[1] + dy - 1 : 0;
-      if (D > 1 && (py < 0 || py >= P.n_cells_d[1])) continue;
-      const int row = nx * (py + P.n_cells_d[1] * pz);
-      const int s0 = ld(P.cell_start + row + x0), s1 = ld(P.cell_start + row + x1 + 1);
-      for (int base = s0; base < s1; base += L) {
-        const int q = base + gl;
-        bool has = false;
-        T t[3] = {(T)0, (T)0, (T)0};
-        if (q < s1 && q != s) {
-          T xj[3], e[3];
-          pos(q, xj);
-          const T s2 = pair_diff<T, D>(xi, xj, e);
-          if (s2 < coef.cut2) {
-            const T dd = sqrt(s2);
-            T F = (T)0;
-            if (dd < coef.rrep) {
-              F = coef.krep * (coef.rrep - dd);
-              has = true;
-            } else if (dd < coef.ratt) {
-              F = coef.from_rep ? -(coef.katt * (dd - coef.rrep)) : -(coef.katt * (coef.ratt - dd));
-              has = true;
-            }
-            if (has) {
-              const T sc = F / dd;
+    // candidate k of the plane: slot off[r] + k of the row r it falls in
+    int off[3] = {0, 0, 0}, end[3] = {0, 0, 0}, total = 0;
 #pragma unroll
-              for (int d = 0; d < D; ++d) t[d] = sc * e[d];
-            }
-          }
-        }
-        // the chunk's terms, added in candidate order by every lane of the group
-#pragma unroll
-        for (int u = 0; u < L; ++u) {
-          const bool hu = __shfl_sync(gmask, has ? 1 : 0, u, L) != 0;
-          T tu[3];
-#pragma unroll
-          for (int d = 0; d < D; ++d) tu[d] = __shfl_sync(gmask, t[d], u, L);
-          if (hu) {
-#pragma unroll
-            for (int d = 0; d < D; ++d) acc[d] = acc[d] + tu[d];
-          }
-        }
+    for (int r = 0; r < ny_rows; ++r) {
+      const int py = D > 1 ? q3[1] + r - 1 : 0;
+      if (D == 1 || (py >= 0 && py < P.n_cells_d[1])) {
+        const int row = nx * (py + P.n_cells_d[1] * pz);
+        const int s0 = start[row + x0];
+        off[r] = s0 - total;
+        total += start[row + x1 + 1] - s0;
       }
+      end[r] = total;
+    }
+    auto slot = [&](int k) {
+      return k + (D == 1 || k < end[0] ? off[0] : (k < end[1] ? off[1] : off[2]));
+    };
+    int qn = gl < total ? slot(gl) : s;
+    T xn[3] = {(T)0, (T)0, (T)0};
+    pos(qn, xn);
+    for (int base = 0; base < total; base += L) {
+      const int q = qn;
+      const T xj[3] = {xn[0], xn[1], xn[2]};
+      if (base + L < total) {
+        qn = base + L + gl < total ? slot(base + L + gl) : s;
+        pos(qn, xn);
+      }
+      T e[3];
+      const T s2 = pair_diff<T, D>(xi, xj, e);
+      T sc = (T)0;
+      if (q != s) {
+        T inv = (T)0;
+        const bool mid = line.mid && s2 > (T)1e-12 && s2 < (T)1e12;
+        const T d = mid ? sqrt_mid(s2, &inv) : sqrt(s2);
+        const bool rep = d < -line.nrrep;
+        const T F = (rep ? line.krep : line.katt) * ((rep ? line.rrep : line.abase) - d);
+        const T f = mid ? div_mid(F, d, inv) : F / d;
+        sc = d < -line.nreach ? f : (T)0;
+      }
+      T t[3];
+#pragma unroll
+      for (int d = 0; d < D; ++d) t[d] = sc != (T)0 ? sc * e[d] : (T)0;
+      // the chunk's terms, added in candidate order by every lane of the group
+#pragma unroll
+      for (int u = 0; u < L; ++u)
+#pragma unroll
+        for (int d = 0; d < D; ++d) acc[d] = acc[d] + __shfl_sync(gmask, t[d], u, L);
     }
   }
-  if (gl == 0) finish_agent<T, D>(P, s, xi, acc);
+  if (gl == 0) finish_agent<T, D>(P, s, xi, acc, x_new);
 }
 
 // nsteps steps; P0 has the parity of the first step, P1 the other one.  The
@@ -172,12 +191,18 @@ __device__ __forceinline__ void small_de(const Params<T>& P, int s) {
 // phase (no thread reads those counters before the next step) so that it
 // stays off the scan's path.
 template <typename T, int D>
-__global__ void __launch_bounds__(kSmallThreads) k_small_steps(Params<T> P0, Params<T> P1,
+__global__ void __launch_bounds__(kSmallMaxThreads) k_small_steps(Params<T> P0, Params<T> P1,
                                                                int nsteps, int n_cells) {
   extern __shared__ int s_start[];  // n_cells + 1 offsets of the grid being built
-  __shared__ int warp_sums[kSmallThreads / 32];
-  const int tid = (int)(blockIdx.x * kSmallThreads + threadIdx.x);
-  const int nth = (int)(gridDim.x * kSmallThreads);
+  __shared__ int warp_sums[kSmallMaxThreads / 32];
+  const int bth = (int)blockDim.x;
+  const int tid = (int)blockIdx.x * bth + (int)threadIdx.x;
+  const int nth = (int)gridDim.x * bth;
+  const PairLine<T> line = make_pair_line<T>(P0.cut2, P0.k_rep, P0.r_rep, P0.k_att, P0.r_att,
+                                             P0.att_form == CBM_ATT_FROM_REP);
+  // every block keeps the offsets of the grid in use
+  for (int c = threadIdx.x; c <= n_cells; c += bth) s_start[c] = P0.cell_start[c];
+  __syncthreads();
   for (int t = 0; t < nsteps; ++t) {
     const Params<T>& P = (t & 1) ? P1 : P0;
     Counters* C = P.ctr;
@@ -188,13 +213,12 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_steps(Params<T> P0, Par
     // Slots are dealt to the blocks in turn (slot s to block s mod blocks),
     // so every block holds agents from all over the community and the dense
     // clumps do not all fall to the same block.
-    const int groups = kSmallThreads / kSmallLanes;
+    const int groups = bth / kSmallLanes;
     for (int s = (int)(threadIdx.x / kSmallLanes) * (int)gridDim.x + (int)blockIdx.x; s < N;
          s += groups * (int)gridDim.x) {
-      small_de<T, D>(P, s);
+      T x[3];
+      small_de<T, D>(P, line, s_start, s, x);
       if ((threadIdx.x & (kSmallLanes - 1)) == 0) {  // k_sort_hist
-        T x[3];
-        to3<T>(P.PB[s], x);
         const int c = cell_of_pos<T, D>(P, x);
         P.s_cell[s] = c;
         P.s_rank[s] = atomicAdd(P.cell_count + c, 1);
@@ -203,18 +227,26 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_steps(Params<T> P0, Par
     cluster_barrier();
     block_scan_counts(P.cell_count, n_cells, s_start, warp_sums);
     if (blockIdx.x == 0)
-      for (int c = threadIdx.x; c <= n_cells; c += kSmallThreads) P.cell_start[c] = s_start[c];
+      for (int c = threadIdx.x; c <= n_cells; c += bth) P.cell_start[c] = s_start[c];
     for (int s = tid; s < N; s += nth) P.s_key[s_start[P.s_cell[s]] + P.s_rank[s]] = P.IB[s];
     cluster_barrier();
     for (int s = tid; s < N; s += nth) {  // stable placement by agent index (k_sort_place)
       const int c = P.s_cell[s];
       const int key = P.IB[s];
+      const typename V4T<T>::type x = P.PB[s];
+      const T v = P.VB[s];
       const int s0 = s_start[c], s1 = s_start[c + 1];
       int r = 0;
-      for (int q = s0; q < s1; ++q) r += P.s_key[q] < key;
+      for (int q = s0; q < s1; q += 4) {  // four keys in flight
+        int k4[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) k4[u] = q + u < s1 ? P.s_key[q + u] : key;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) r += k4[u] < key;
+      }
       const int ns = s0 + r;
-      P.PA[ns] = P.PB[s];
-      P.VA[ns] = P.VB[s];
+      P.PA[ns] = x;
+      P.VA[ns] = v;
       P.IA[ns] = key;
       P.inv[key] = ns;
       P.cell_of_slot[ns] = c;
