@@ -929,9 +929,12 @@ int flags_to_status(int err) {
   return CBM_OK;
 }
 
+// the counters after all that is enqueued: one copy to page-locked memory and
+// one wait
 int read_counters(cbm_ctx* c, Counters* h) {
+  CUDA_TRY(c, cudaMemcpyAsync(c->h_ctr, c->ctr, sizeof(Counters), cudaMemcpyDeviceToHost, c->stream));
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-  CUDA_TRY(c, cudaMemcpy(h, c->ctr, sizeof(Counters), cudaMemcpyDeviceToHost));
+  *h = *c->h_ctr;
   return CBM_OK;
 }
 
@@ -1208,6 +1211,27 @@ static __global__ void k_default_ids(long long* id, int n) {
   if (i < n) id[i] = (long long)i + 1;
 }
 
+// Ranges of words to clear: the absent fields of an upload and the rows beyond N.
+struct ClearList {
+  unsigned* at[12];
+  long long words[12];
+  int n;
+};
+static __global__ void __launch_bounds__(kTile) k_clear(ClearList L) {
+  for (int k = 0; k < L.n; ++k)
+    for (long long i = (long long)blockIdx.x * kTile + threadIdx.x; i < L.words[k];
+         i += (long long)gridDim.x * kTile)
+      L.at[k][i] = 0u;
+}
+
+// An upload's counters; the epochs go on from those they replace, so that
+// stale tile states never match.
+static __global__ void k_load_counters(Counters* C, Counters h) {
+  h.scan_epoch = C->scan_epoch + 1u;
+  h.fate_epoch = C->fate_epoch + 1u;
+  *C = h;
+}
+
 int cbm_upload(cbm_ctx* c, const cbm_state_view* h) {
   if (!c || !h) return fail(c, CBM_ERR_ARG, "null argument");
   cudaSetDevice(c->device);
@@ -1218,23 +1242,19 @@ int cbm_upload(cbm_ctx* c, const cbm_state_view* h) {
   for (int d = 0; d < k.dims; ++d)
     if (N && !h->pos[d]) return fail(c, CBM_ERR_ARG, "pos[%d] is NULL", d);
   if (k.growth && N && (!h->v || !h->g)) return fail(c, CBM_ERR_ARG, "growth needs v and g");
-  CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   cudaStream_t st = c->stream;
-  // the epochs of the counters being replaced, read before anything is
-  // enqueued, so that the copies, the counters and the first sort follow one
-  // another with one synchronisation at the end
-  Counters old;
-  CUDA_TRY(c, cudaMemcpy(&old, c->ctr, sizeof old, cudaMemcpyDeviceToHost));
   // staging: index order; absent fields are zeros (loadToPlatform! pads with
   // zeros), and so is every field beyond N.  A field given by the caller is
   // copied into [0, N) and cleared beyond it only.
+  // (one kernel clears all of them)
+  ClearList clear{};
   auto stage = [&](void* dst, const void* src, size_t elem) -> cudaError_t {
     const size_t from = (src && N) ? N : 0;
-    cudaError_t e = cudaSuccess;
-    if (from) e = cudaMemcpyAsync(dst, src, N * elem, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && nm > from)
-      e = cudaMemsetAsync((char*)dst + from * elem, 0, (nm - from) * elem, st);
-    return e;
+    if (nm > from) {
+      clear.at[clear.n] = (unsigned*)((char*)dst + from * elem);
+      clear.words[clear.n++] = (long long)((nm - from) * (elem / 4));
+    }
+    return from ? cudaMemcpyAsync(dst, src, N * elem, cudaMemcpyHostToDevice, st) : cudaSuccess;
   };
   for (int d = 0; d < 3; ++d) {
     CUDA_TRY(c, stage(c->hx[d], d < k.dims ? h->pos[d] : nullptr, S));
@@ -1245,6 +1265,7 @@ int cbm_upload(cbm_ctx* c, const cbm_state_view* h) {
   CUDA_TRY(c, stage(c->PAR, h->parent, 8));
   // ids: the caller's (copied straight from its array), else 1..N; zero beyond N
   CUDA_TRY(c, stage(c->ID, h->id, 8));
+  k_clear<<<2 * c->n_sm, kTile, 0, st>>>(clear);
   if (N && !h->id) k_default_ids<<<grid_blocks((long long)N), kTile, 0, st>>>(c->ID, (int)N);
   if (k.medium) {
     const size_t nb = (size_t)c->n_nodes * S;
@@ -1273,10 +1294,7 @@ int cbm_upload(cbm_ctx* c, const cbm_state_view* h) {
   hc.id_max = h->id_max > 0 ? h->id_max : h->N;
   hc.slots = h->N;
   hc.resort = 1;  // flagRecomputeNeighbors_ = [1] and computeNeighbors! at load (communityStructure.jl:480,648)
-  hc.scan_epoch = old.scan_epoch + 1;  // keep the epoch monotonic so stale tile states never match
-  hc.fate_epoch = old.fate_epoch + 1;
-  *c->h_ctr = hc;  // pinned: the copy is ordered on the stream, without a wait
-  CUDA_TRY(c, cudaMemcpyAsync(c->ctr, c->h_ctr, sizeof hc, cudaMemcpyHostToDevice, st));
+  k_load_counters<<<1, 1, 0, st>>>(c->ctr, hc);
   c->parity = 0;
   reset_stage_flags(c);
   c->loaded = true;
