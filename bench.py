@@ -201,12 +201,12 @@ class SmiClocks:
                 "samples": len(sm), "source": "nvidia-smi -lms 200"}
 
 
-# Per-agent figures of one ncu capture of k_agent_de on the grown colony
+# Per-agent figures of one ncu capture of k_agent_de_tile on the grown colony
 # (Float32): DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) and warp
 # instructions (smsp__inst_executed.sum) per agent of the launch.  They are
 # read from the capture's summary under profiles/, which gives the command
 # that made it; a changed kernel needs a new capture.
-KERNEL_PROFILE = os.path.join(ROOT, "profiles", "k_agent_de_grown_colony_1m_f32.md")
+KERNEL_PROFILE = os.path.join(ROOT, "profiles", "k_agent_de_tile_grown_colony_1m_f32.md")
 
 
 def profile_per_agent(path=KERNEL_PROFILE):
@@ -227,7 +227,7 @@ def profile_per_agent(path=KERNEL_PROFILE):
 def alg_bytes_per_agent(name, s, d, nbar, verlet, fate):
     """Compulsory HBM bytes per agent of one launch (neighbor-position gathers,
     which are served from L2, are not counted)."""
-    if name == "k_agent_de":
+    if name in ("k_agent_de", "k_agent_de_tile"):
         b = 2 * d * s + 2 * s + s  # positions r/w, volume r/w, growth rate
         b += (4 + 4 * nbar) if verlet else 8  # list count + entries, or own cell range
         b += d * s if verlet else 0  # displacement check against posOld
@@ -439,7 +439,7 @@ def run_ours(args, rank, world, local_rank):
     if bpa is not None:
         avg_ms = stats[top][0]
         achieved = bpa * agents / (avg_ms / 1e3) / 1e9
-        per = profile_per_agent() if (top == "k_agent_de" and s == 4 and walked
+        per = profile_per_agent() if (top == "k_agent_de_tile" and s == 4 and walked
                                       and args.workload == "grown") else {}
         traffic = per.get("dram_bytes_per_agent")
         roof = {"kernel": top, "bound": "hbm", "achieved": round(achieved, 1),
