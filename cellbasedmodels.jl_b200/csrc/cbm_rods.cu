@@ -16,16 +16,21 @@
 // The state is double-buffered: k_rod_step reads buffer a (committed) and
 // writes buffer b, so 1 and 2 are one launch and the commit is a swap.  The
 // same launch computes the cell of each new position and its atomic rank
-// (assignCells); the scan, scatter and stable passes of cbm_grid.cuh finish
-// the grid.  Four launches per step (seven with growth: the division flags,
+// (assignCells); the scan, scatter and placement passes finish the
+// grid.  Four launches per step (seven with growth: the division flags,
 // their scan and the holes come first), replayed from a CUDA graph of two
 // steps.
 //
-// A rod's candidates are spread over a group of kRodLanes lanes: lane k takes
-// candidates k, k + G, ...; after each chunk of G the group's terms are
-// broadcast by shuffles and every lane adds them in candidate order, so the
-// sums have the reference's order.  Only contacts add (a pair without contact
-// contributes +0.0, which leaves a sum started at +0.0 unchanged).
+// A rod's candidates are spread over a group of 4, 8 or 16 lanes, which keep
+// those that may touch it (cbm_rod_apart, a tenth of the contact force's work)
+// in order; the block's threads then take the kept pairs of all its rods, and
+// the terms of each rod are added in candidate order.  Only contacts add (a
+// pair without contact contributes +0.0, which leaves a sum started at +0.0
+// unchanged).  What a candidate shows is read from copies in cell order.
+// Bound by latency: Float64 sequences on about 7 warps a scheduler.  32768
+// rods, Float64: 81.5 -> 51.3 us a step (24 of them the grid's three kernels);
+// the filter alone, with candidates read by index, 78.9; with cell order 61.4
+// with eight lanes.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -41,11 +46,8 @@ using namespace cbm;
 namespace {
 
 constexpr int kRodBlock = 128;
-#ifndef CBM_ROD_LANES
-#define CBM_ROD_LANES 8
-#endif
-constexpr int kRodLanes = CBM_ROD_LANES;  // lanes per rod
-static_assert(kRodLanes == 4 || kRodLanes == 8 || kRodLanes == 16, "lanes per rod");
+// Candidates a rod holds for the contact force, by its lanes
+constexpr int rod_queue(int lanes) { return lanes == 16 ? 32 : 24; }
 
 // the per-rod arrays that a step rewrites; d, l, m are constant in rods2D and
 // single arrays, while rods2dGrowth rewrites (moves) every field, so there
@@ -56,13 +58,18 @@ enum {
 };
 constexpr int kPlainArrays = kSL;  // arrays of the rods2D state
 
+// what a rod shows its neighbors, in the order of the walk
+enum { kQX = 0, kQY, kQCOS, kQSIN, kQL, kQD, kQVX, kQVY, kQM, kSeenArrays };
+template <typename T>
+struct RodSeen {
+  T* q[kSeenArrays];
+};
+
 template <typename T>
 struct RodStep {
   T* a[kStateArrays];  // committed
   T* b[kStateArrays];  // written
-  const T* d;
-  const T* l;
-  const T* m;
+  RodSeen<const T> seen;  // of a, in cell order (all pairs: index order, a itself)
   const int* cell_start;  // grid of a
   const int* cell_agents;
   int* cell_count;        // zero on entry (the scan clears it)
@@ -94,11 +101,6 @@ __global__ void __launch_bounds__(kTile) k_rod_geom(T* const* a, int n) {
   cbm_rod_cossin<T>(a[kSTH][i], &c, &s);
   a[kSCOS][i] = c;
   a[kSSIN][i] = s;
-}
-
-template <typename T>
-__device__ __forceinline__ T shfl_group(T v, int q) {
-  return __shfl_sync(0xffffffffu, v, q, kRodLanes);
 }
 
 // assignCells for a row of b (neighbors.jl:763-821)
@@ -168,84 +170,13 @@ __device__ void rod_divide(const RodStep<T>& R, int i, int n) {
   }
 }
 
-// Steps 1 and 2 of one step (rods.jl:86-118 with rodForces, :21-59), and the
-// cell assignment of step 3 (assignCells, neighbors.jl:763-821)
+// The update of the rod at `slot` of the walk with the sums of its contacts
 template <typename T, bool GROW>
-__global__ void __launch_bounds__(kRodBlock) k_rod_step(RodStep<T> R) {
-  pdl_wait();
-  const int t = blockIdx.x * kRodBlock + threadIdx.x;
-  const int i = t / kRodLanes, lane = t % kRodLanes;
-  const int n = GROW ? (int)R.cnt_a[0] : R.n;
-  const bool live = i < n;
-  if (t == 0 && !R.full) {
-    R.ctr->scan_ticket = 0u;  // fresh tickets and tile-state generation for the scan
-    R.ctr->scan_epoch = R.ctr->scan_epoch + 1u;
-  }
-  CbmRodGeom<T> g{(T)0, (T)0, (T)1, (T)0, (T)0};
-  T d1 = (T)0, m1 = (T)1, vx1 = (T)0, vy1 = (T)0;
-  if (live) {
-    g = CbmRodGeom<T>{R.a[kSX][i], R.a[kSY][i], R.a[kSCOS][i], R.a[kSSIN][i], R.l[i]};
-    d1 = R.d[i];
-    m1 = R.m[i];
-    vx1 = R.a[kSVX][i];
-    vy1 = R.a[kSVY][i];
-  }
-  // candidate runs: all rods, or the three rows of x-neighbor cells
-  int rs[3] = {0, 0, 0}, re[3] = {0, 0, 0};
-  if (live) {
-    if (R.full) {
-      re[0] = n;
-    } else {
-      const T x[2] = {g.x, g.y};
-      const int c = cell_of<T, 2>(R.edge, R.box_lo, R.box_hi, R.n_cells_d, x);
-      const int nx = R.n_cells_d[0], ny = R.n_cells_d[1];
-      const int qx = c % nx, qy = c / nx;
-      const int x0 = qx > 0 ? qx - 1 : 0, x1 = qx < nx - 1 ? qx + 1 : nx - 1;
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        const int py = qy + r - 1;
-        if (py < 0 || py >= ny) continue;
-        rs[r] = R.cell_start[nx * py + x0];
-        re[r] = R.cell_start[nx * py + x1 + 1];
-      }
-    }
-  }
-  const int group_shift = (threadIdx.x & 31) & ~(kRodLanes - 1);
-  T fx = (T)0, fy = (T)0, w = (T)0, p = (T)0;
-#pragma unroll 1
-  for (int r = 0; r < 3; ++r) {
-    const int chunks = __reduce_max_sync(0xffffffffu, (re[r] - rs[r] + kRodLanes - 1) / kRodLanes);
-#pragma unroll 1
-    for (int c = 0; c < chunks; ++c) {
-      const int s = rs[r] + c * kRodLanes + lane;
-      bool hit = false;
-      T gx = (T)0, gy = (T)0, gw = (T)0, gp = (T)0;
-      if (s < re[r]) {
-        const int j = R.full ? s : R.cell_agents[s];
-        if (j != i) {
-          const CbmRodGeom<T> h{R.a[kSX][j], R.a[kSY][j], R.a[kSCOS][j], R.a[kSSIN][j], R.l[j]};
-          hit = cbm_rod_forces<T>(g, d1, vx1, vy1, m1, h, R.d[j], R.a[kSVX][j], R.a[kSVY][j], R.k,
-                                  &gx, &gy, &gw);
-          if (hit) gp = sqrt(gx * gx + gy * gy);
-        }
-      }
-      const unsigned hits = __ballot_sync(0xffffffffu, hit);
-      if (hits == 0u) continue;
-      const unsigned mine = (hits >> group_shift) & ((1u << kRodLanes) - 1u);
-#pragma unroll
-      for (int q = 0; q < kRodLanes; ++q) {
-        const T ax = shfl_group(gx, q), ay = shfl_group(gy, q);
-        const T aw = shfl_group(gw, q), ap = shfl_group(gp, q);
-        if (mine & (1u << q)) {
-          fx = fx + ax;
-          fy = fy + ay;
-          w = w + aw;
-          p = p + ap;
-        }
-      }
-    }
-  }
-  if (!live || lane != 0) return;
+__device__ __forceinline__ void finish_rod(const RodStep<T>& R, int slot, int n, T fx, T fy, T w,
+                                           T p) {
+  if (slot >= n) return;
+  const RodSeen<const T>& Q = R.seen;
+  const int i = R.full ? slot : R.cell_agents[slot];
   int row = i;  // the final row of rod i
   if constexpr (GROW) {
     if (R.div_rank[i + 1] != R.div_rank[i]) {
@@ -262,13 +193,14 @@ __global__ void __launch_bounds__(kRodBlock) k_rod_step(RodStep<T> R) {
   }
   // Euler: u + du dt with the committed forces, then the commit of the sums
   const T dt = R.dt;
-  const T vx = vx1, vy = vy1, om = R.a[kSOM][i], th = R.a[kSTH][i];
-  const T d = d1, l = g.l, m = m1;
+  const T x = Q.q[kQX][slot], y = Q.q[kQY][slot], vx = Q.q[kQVX][slot], vy = Q.q[kQVY][slot];
+  const T d = Q.q[kQD][slot], l = Q.q[kQL][slot], m = Q.q[kQM][slot];
+  const T om = R.a[kSOM][i], th = R.a[kSTH][i];
   const T dvx = -R.beta * vx + R.a[kSFX][i] / m;
   const T dvy = -R.beta * vy + R.a[kSFY][i] / m;
   const T den = (m * ((d + l) * (d + l))) / (T)12 + m * (d * d);
   const T dom = R.a[kSW][i] / den - R.beta_w * om;
-  const T xn = g.x + vx * dt, yn = g.y + vy * dt, thn = th + om * dt;
+  const T xn = x + vx * dt, yn = y + vy * dt, thn = th + om * dt;
   R.b[kSX][row] = xn;
   R.b[kSY][row] = yn;
   R.b[kSVX][row] = vx + dvx * dt;
@@ -291,6 +223,130 @@ __global__ void __launch_bounds__(kRodBlock) k_rod_step(RodStep<T> R) {
     R.b[kSM][row] = m;
   }
   if (!R.full) rod_assign_cell<T>(R, row, xn, yn);
+}
+
+// Steps 1 and 2 of one step (rods.jl:86-118 with rodForces, :21-59), and the
+// cell assignment of step 3 (assignCells, neighbors.jl:763-821)
+template <typename T, bool GROW, int kRodLanes>
+__global__ void __launch_bounds__(kRodBlock) k_rod_step(RodStep<T> R) {
+  pdl_wait();
+  const int t = blockIdx.x * kRodBlock + threadIdx.x;
+  const int slot = t / kRodLanes, lane = t % kRodLanes;  // one group a place of the walk
+  const int n = GROW ? (int)R.cnt_a[0] : R.n;
+  const bool live = slot < n;
+  if (t == 0 && !R.full) {
+    R.ctr->scan_ticket = 0u;  // fresh tickets and tile-state generation for the scan
+    R.ctr->scan_epoch = R.ctr->scan_epoch + 1u;
+  }
+  const RodSeen<const T>& Q = R.seen;
+  auto geom = [&](int s) {
+    return CbmRodGeom<T>{Q.q[kQX][s], Q.q[kQY][s], Q.q[kQCOS][s], Q.q[kQSIN][s], Q.q[kQL][s]};
+  };
+  CbmRodGeom<T> g{(T)0, (T)0, (T)1, (T)0, (T)0};
+  T d1 = (T)0;
+  if (live) {
+    g = geom(slot);
+    d1 = Q.q[kQD][slot];
+  }
+  // candidate runs: all rods, or the three rows of x-neighbor cells
+  int rs[3] = {0, 0, 0}, re[3] = {0, 0, 0};
+  if (live) {
+    if (R.full) {
+      re[0] = n;
+    } else {
+      const T x[2] = {g.x, g.y};
+      const int c = cell_of<T, 2>(R.edge, R.box_lo, R.box_hi, R.n_cells_d, x);
+      const int nx = R.n_cells_d[0], ny = R.n_cells_d[1];
+      const int qx = c % nx, qy = c / nx;
+      const int x0 = qx > 0 ? qx - 1 : 0, x1 = qx < nx - 1 ? qx + 1 : nx - 1;
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        const int py = qy + r - 1;
+        if (py < 0 || py >= ny) continue;
+        rs[r] = R.cell_start[nx * py + x0];
+        re[r] = R.cell_start[nx * py + x1 + 1];
+      }
+    }
+  }
+  // Filter, force and sum in turn.  A rod's group tests its candidates
+  // kRodLanes at a time with cbm_rod_apart and queues those it cannot rule
+  // out (about a sixth), in order.  The block's threads then take the queued
+  // pairs of all its rods, one each, so that the contact force, the long
+  // serial part, runs on full warps; and four threads a rod add the terms of
+  // its pairs in candidate order, one component each.  A queue without room
+  // ends a turn early.
+  constexpr int kRods = kRodBlock / kRodLanes, kRodQueue = rod_queue(kRodLanes);
+  static_assert(kRods <= 32 && 4 * kRods <= kRodBlock, "one warp scans the counts, four threads sum");
+  __shared__ int queue[kRodQueue * kRods];
+  __shared__ unsigned char rod_of[kRodQueue * kRods];  // of pair k of the turn
+  __shared__ int count[kRods], first[kRods];
+  __shared__ T term[kRodQueue * kRods][4];
+  __shared__ T sums[4][kRods];
+  const int grp = threadIdx.x / kRodLanes, lane32 = threadIdx.x & 31;
+  const int base = blockIdx.x * kRods;
+  const int group_shift = lane32 & ~(kRodLanes - 1);
+  constexpr unsigned kGroup = (1u << kRodLanes) - 1u;
+  const int n0 = re[0] - rs[0], n01 = n0 + (re[1] - rs[1]), total = n01 + (re[2] - rs[2]);
+  const int chunks = __reduce_max_sync(0xffffffffu, (total + kRodLanes - 1) / kRodLanes);
+  T sum = (T)0;  // threads below 4 * kRods: component threadIdx.x % 4 of rod threadIdx.x / 4
+  int c = 0;
+  for (;;) {
+    int nq = 0;
+    for (bool room = true; room && c < chunks; ++c) {
+      const int q = c * kRodLanes + lane;
+      bool keep = false;
+      int s = 0;
+      if (q < total) {
+        s = q < n0 ? rs[0] + q : q < n01 ? rs[1] + (q - n0) : rs[2] + (q - n01);
+        keep = s != slot && !cbm_rod_apart<T>(g, d1, geom(s), Q.q[kQD][s]);
+      }
+      const unsigned kept = (__ballot_sync(0xffffffffu, keep) >> group_shift) & kGroup;
+      if (keep) queue[grp * kRodQueue + nq + __popc(kept & ((1u << lane) - 1u))] = s;
+      nq += __popc(kept);
+      room = !__any_sync(0xffffffffu, nq > kRodQueue - kRodLanes);
+    }
+    if (lane == 0) count[grp] = nq;
+    const bool more = __syncthreads_or(c < chunks);
+    // every warp scans the counts
+    const int own = lane32 < kRods ? count[lane32] : 0;
+    int upto = own;
+#pragma unroll
+    for (int o = 1; o < 32; o *= 2) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane32 >= o) upto += v;
+    }
+    const int pairs = __shfl_sync(0xffffffffu, upto, 31);
+    const int start = __shfl_sync(0xffffffffu, upto - own, grp);
+    if (threadIdx.x < kRods) first[threadIdx.x] = upto - own;
+    for (int k = lane; k < nq; k += kRodLanes) rod_of[start + k] = (unsigned char)grp;
+    __syncthreads();
+    for (int k = threadIdx.x; k < pairs; k += kRodBlock) {
+      const int r = rod_of[k], s = queue[r * kRodQueue + (k - first[r])], o = base + r;
+      T gx = (T)0, gy = (T)0, gw = (T)0, gp = (T)0;
+      // a pair without contact adds +0.0, which leaves a sum begun at +0.0 as it is
+      if (cbm_rod_forces<T>(geom(o), Q.q[kQD][o], Q.q[kQVX][o], Q.q[kQVY][o], Q.q[kQM][o], geom(s),
+                            Q.q[kQD][s], Q.q[kQVX][s], Q.q[kQVY][s], R.k, &gx, &gy, &gw))
+        gp = sqrt(gx * gx + gy * gy);
+      term[k][0] = gx;
+      term[k][1] = gy;
+      term[k][2] = gw;
+      term[k][3] = gp;
+    }
+    __syncthreads();
+    if (threadIdx.x < 4 * kRods) {
+      const int r = threadIdx.x >> 2, k0 = first[r], k1 = k0 + count[r];
+      for (int k = k0; k < k1; ++k) sum = sum + term[k][threadIdx.x & 3];
+    }
+    if (!more) break;
+    __syncthreads();  // what this turn wrote is read before the next overwrites it
+  }
+  if (threadIdx.x < 4 * kRods) sums[threadIdx.x & 3][threadIdx.x >> 2] = sum;
+  __syncthreads();
+  // one thread a rod: done by each group's first lane the update would keep a
+  // warp busy for 32 / kRodLanes rods
+  if (threadIdx.x >= kRods) return;
+  finish_rod<T, GROW>(R, base + threadIdx.x, n, sums[0][threadIdx.x], sums[1][threadIdx.x],
+                      sums[2][threadIdx.x], sums[3][threadIdx.x]);
 }
 
 // rods2dGrowth, before the step: the division flags l > lTarget of the
@@ -322,7 +378,7 @@ __global__ void __launch_bounds__(kTile) k_rod_holes(RodStep<T> R, int* holes, C
   if (R.div_rank[i + 1] != R.div_rank[i]) holes[R.div_rank[i]] = i;
 }
 
-// k_grid_scatter / k_grid_stable of cbm_grid.cuh with the rod count on the device
+// k_grid_scatter of cbm_grid.cuh with the rod count on the device
 template <typename T>
 __global__ void __launch_bounds__(kTile) k_rod_scatter(GridParams<T> G, const long long* cnt) {
   pdl_wait();
@@ -331,16 +387,27 @@ __global__ void __launch_bounds__(kTile) k_rod_scatter(GridParams<T> G, const lo
   G.cell_tmp[G.cell_start[G.agent_cell[i]] + G.agent_rank[i]] = i;
 }
 
+// k_grid_stable of cbm_grid.cuh, with what each rod shows its neighbors put in
+// cell order beside it.  Rods keep their index order, in which neighbors in
+// space lie anywhere: read by index, every value of every candidate was a
+// sector of its own (32768 rods of 38 candidates: 240 MB a step through L1 and
+// L2).  `cnt`: the rod count on the device (null: G.n).
 template <typename T>
-__global__ void __launch_bounds__(kTile) k_rod_stable(GridParams<T> G, const long long* cnt) {
+__global__ void __launch_bounds__(kTile) k_rod_place(GridParams<T> G, const long long* cnt,
+                                                     RodSeen<const T> from, RodSeen<T> to) {
   pdl_wait();
   const int i = blockIdx.x * kTile + threadIdx.x;
-  if (i >= (int)cnt[0]) return;
+  if (i >= (cnt ? (int)cnt[0] : G.n)) return;
+  T v[kSeenArrays];
+#pragma unroll
+  for (int k = 0; k < kSeenArrays; ++k) v[k] = from.q[k][i];
   const int c = G.agent_cell[i];
   const int s0 = G.cell_start[c], s1 = G.cell_start[c + 1];
   int r = 0;
   for (int s = s0; s < s1; ++s) r += ld(G.cell_tmp + s) < i;
   G.cell_agents[s0 + r] = i;
+#pragma unroll
+  for (int k = 0; k < kSeenArrays; ++k) to.q[k][s0 + r] = v[k];
 }
 
 }  // namespace
@@ -350,6 +417,7 @@ struct cbm_rods {
   int tsize = 4;
   cudaStream_t stream = nullptr;
   int n = 0;
+  long long resident = 0;            // threads of the step kernel held at once
   int cur = 0;                       // buffer holding the committed state
   void* st[2][kStateArrays] = {};    // double-buffered per-rod arrays
   void* dlm[3] = {};                 // d, l, m
@@ -364,6 +432,7 @@ struct cbm_rods {
   int* agent_rank = nullptr;
   int* cell_tmp = nullptr;
   int* cell_agents = nullptr;
+  void* seen[kSeenArrays] = {};      // in cell order
   unsigned long long* scan_state = nullptr;
   // rods2dGrowth: {n, step} per buffer on the device, the division ranks
   bool grow = false;
@@ -408,6 +477,8 @@ void rfree(cbm_rods* r) {
     for (void*& p : b)
       if (p) cudaFree(p), p = nullptr;
   for (void*& p : r->dlm)
+    if (p) cudaFree(p), p = nullptr;
+  for (void*& p : r->seen)
     if (p) cudaFree(p), p = nullptr;
   for (void* p : {(void*)r->ptrs, (void*)r->ctr, (void*)r->cell_count, (void*)r->cell_start,
                   (void*)r->agent_cell, (void*)r->agent_rank, (void*)r->cell_tmp,
@@ -467,6 +538,22 @@ GridParams<T> grid_params(const cbm_rods* r) {
   return G;
 }
 
+// what the rods of buffer `buf` show, in index order
+template <typename T>
+RodSeen<const T> seen_by_index(const cbm_rods* r, int buf) {
+  void* const* st = r->st[buf];
+  return RodSeen<const T>{{(const T*)st[kSX], (const T*)st[kSY], (const T*)st[kSCOS],
+                           (const T*)st[kSSIN], (const T*)(r->grow ? st[kSL] : r->dlm[1]),
+                           (const T*)(r->grow ? st[kSD] : r->dlm[0]), (const T*)st[kSVX],
+                           (const T*)st[kSVY], (const T*)(r->grow ? st[kSM] : r->dlm[2])}};
+}
+template <typename T>
+RodSeen<T> seen_by_cell(const cbm_rods* r) {
+  RodSeen<T> S;
+  for (int k = 0; k < kSeenArrays; ++k) S.q[k] = (T*)r->seen[k];
+  return S;
+}
+
 // computeNeighbors! from scratch on the committed positions (after upload)
 template <typename T>
 void enqueue_full_grid(cbm_rods* r) {
@@ -475,7 +562,40 @@ void enqueue_full_grid(cbm_rods* r) {
   k_grid_hist<T, 2><<<nb, kTile, 0, r->stream>>>(G);
   k_scan_cells<<<G.n_scan_tiles, kTile, 0, r->stream>>>(grid_scan_args(G));
   k_grid_scatter<T><<<nb, kTile, 0, r->stream>>>(G);
-  k_grid_stable<T><<<nb, kTile, 0, r->stream>>>(G);
+  k_rod_place<T><<<nb, kTile, 0, r->stream>>>(G, nullptr, seen_by_index<T>(r, r->cur),
+                                              seen_by_cell<T>(r));
+}
+
+template <typename T, bool GROW, int kLanes>
+void launch_rod_step_lanes(cbm_rods* r, const RodStep<T>& R, long long n, bool pdl) {
+  const unsigned nb = (unsigned)((n * kLanes + kRodBlock - 1) / kRodBlock);
+  launch_serial(r->stream, pdl, k_rod_step<T, GROW, kLanes>, dim3(nb), dim3(kRodBlock), 0, R);
+}
+// Lanes a rod: the most with which the blocks of all rods are resident at
+// once, four beyond that.  Few rods leave the chip idle and each rod's serial
+// candidates bound the step; many rods pay for every lane's share of the setup
+// (us a step, Float64, 16 / 8 / 4 lanes: 2500 rods 20.2 / 23.3 / 27.6, 9500
+// 35.2 / 30.4 / 31.0, 32768 74.8 / 61.5 / 51.3; Float32, whose blocks need half
+// the registers: 5000 20.5 / 22.5 / 26.0, 14000 30.0 / 25.6 / 28.4, 32768 45.9
+// / 38.0 / 34.4).  A growing colony passes through several sizes in one
+// graph: sixteen when its capacity fits, four when its start does not fit
+// with eight.  The sums do not depend on it.
+template <typename T, bool GROW>
+void launch_rod_step(cbm_rods* r, const RodStep<T>& R, long long n, bool pdl) {
+  if (n * 16 <= r->resident) launch_rod_step_lanes<T, GROW, 16>(r, R, n, pdl);
+  else if ((long long)r->n * 8 <= r->resident) launch_rod_step_lanes<T, GROW, 8>(r, R, n, pdl);
+  else launch_rod_step_lanes<T, GROW, 4>(r, R, n, pdl);
+}
+// threads of k_rod_step that the device holds at once
+template <typename T, bool GROW>
+long long rod_resident() {
+  int dev = 0, sm = 0, blocks = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_rod_step<T, GROW, 8>, kRodBlock,
+                                                    0) != cudaSuccess)
+    return 0;
+  return (long long)sm * blocks * kRodBlock;
 }
 
 template <typename T>
@@ -487,9 +607,6 @@ void enqueue_rod_step(cbm_rods* r) {
     R.a[q] = (T*)r->st[r->cur][q];
     R.b[q] = (T*)r->st[1 - r->cur][q];
   }
-  R.d = (const T*)(r->grow ? r->st[r->cur][kSD] : r->dlm[0]);
-  R.l = (const T*)(r->grow ? r->st[r->cur][kSL] : r->dlm[1]);
-  R.m = (const T*)(r->grow ? r->st[r->cur][kSM] : r->dlm[2]);
   R.cell_start = r->cell_start;
   R.cell_agents = r->cell_agents;
   R.cell_count = r->cell_count;
@@ -498,6 +615,13 @@ void enqueue_rod_step(cbm_rods* r) {
   R.ctr = r->ctr;
   R.n = r->n;
   R.full = k.neighbors == CBM_NEIGH_FULL;
+  if (R.full) {
+    const RodSeen<const T> S = seen_by_index<T>(r, r->cur);
+    for (int q = 0; q < kSeenArrays; ++q) R.seen.q[q] = S.q[q];
+  } else {
+    const RodSeen<T> S = seen_by_cell<T>(r);
+    for (int q = 0; q < kSeenArrays; ++q) R.seen.q[q] = S.q[q];
+  }
   for (int d = 0; d < 2; ++d) {
     R.box_lo[d] = (T)k.box_lo[d];
     R.box_hi[d] = (T)k.box_hi[d];
@@ -509,9 +633,7 @@ void enqueue_rod_step(cbm_rods* r) {
   R.beta_w = (T)k.beta_w;
   R.k = CbmRodCoef<T>{(T)k.kn, (T)k.gamma_n, (T)k.gamma_t, (T)k.mu_cc};
   if (!r->grow) {
-    const long long threads = (long long)(r->n > 0 ? r->n : 1) * kRodLanes;
-    const unsigned nb = (unsigned)((threads + kRodBlock - 1) / kRodBlock);
-    k_rod_step<T, false><<<nb, kRodBlock, 0, r->stream>>>(R);
+    launch_rod_step<T, false>(r, R, r->n > 0 ? r->n : 1, false);
     r->cur = 1 - r->cur;
     if (!R.full) {
       // the rest of computeNeighbors! on the new positions
@@ -521,7 +643,8 @@ void enqueue_rod_step(cbm_rods* r) {
       launch_serial(r->stream, true, k_scan_cells, dim3(G.n_scan_tiles), dim3(kTile), 0,
                     grid_scan_args(G));
       launch_serial(r->stream, true, k_grid_scatter<T>, dim3(ng), dim3(kTile), 0, G);
-      launch_serial(r->stream, true, k_grid_stable<T>, dim3(ng), dim3(kTile), 0, G);
+      launch_serial(r->stream, true, k_rod_place<T>, dim3(ng), dim3(kTile), 0, G,
+                    (const long long*)nullptr, seen_by_index<T>(r, r->cur), seen_by_cell<T>(r));
     }
     return;
   }
@@ -549,9 +672,7 @@ void enqueue_rod_step(cbm_rods* r) {
   // from here each kernel follows a kernel on the stream: programmatic launches
   launch_serial(r->stream, true, k_scan_cells, dim3(A.n_tiles), dim3(kTile), 0, A);
   launch_serial(r->stream, true, k_rod_holes<T>, dim3(nt), dim3(kTile), 0, R, r->holes, r->ctr);
-  const long long threads = (long long)k.n_max * kRodLanes;
-  const unsigned nb = (unsigned)((threads + kRodBlock - 1) / kRodBlock);
-  launch_serial(r->stream, true, k_rod_step<T, true>, dim3(nb), dim3(kRodBlock), 0, R);
+  launch_rod_step<T, true>(r, R, k.n_max, true);
   r->cur = 1 - r->cur;
   if (!R.full) {
     const GridParams<T> G = grid_params<T>(r);
@@ -559,7 +680,8 @@ void enqueue_rod_step(cbm_rods* r) {
     launch_serial(r->stream, true, k_scan_cells, dim3(G.n_scan_tiles), dim3(kTile), 0,
                   grid_scan_args(G));
     launch_serial(r->stream, true, k_rod_scatter<T>, dim3(nt), dim3(kTile), 0, G, cnt);
-    launch_serial(r->stream, true, k_rod_stable<T>, dim3(nt), dim3(kTile), 0, G, cnt);
+    launch_serial(r->stream, true, k_rod_place<T>, dim3(nt), dim3(kTile), 0, G, cnt,
+                  seen_by_index<T>(r, r->cur), seen_by_cell<T>(r));
   }
 }
 
@@ -639,9 +761,13 @@ int cbm_rods_create(cbm_rods** out, const cbm_rods_config* cfg) {
     }
     r->n_cells = (int)nc;
   }
+  r->resident = r->tsize == 8 ? (r->grow ? rod_resident<double, true>() : rod_resident<double, false>())
+                              : (r->grow ? rod_resident<float, true>() : rod_resident<float, false>());
   const size_t n = (size_t)k.n_max, S = (size_t)r->tsize;
   bool ok = cudaStreamCreateWithFlags(&r->stream, cudaStreamNonBlocking) == cudaSuccess;
   const int arrays = r->grow ? kStateArrays : kPlainArrays;
+  if (k.neighbors == CBM_NEIGH_CELL_LINKED)
+    for (void*& p : r->seen) ok = ok && cudaMalloc(&p, n * S) == cudaSuccess;
   for (auto& b : r->st)
     for (int q = 0; q < arrays; ++q) ok = ok && cudaMalloc(&b[q], n * S) == cudaSuccess;
   if (!r->grow)

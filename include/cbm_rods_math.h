@@ -198,4 +198,36 @@ CBM_HD bool cbm_rod_forces(const CbmRodGeom<T>& a, T d1, T vx1, T vy1, T m1,
   return true;
 }
 
+/* True only where cbm_rod_forces(a, d1, .., b, d2, ..) finds no contact, at a
+ * tenth of its work: no square root and no quotient.
+ *
+ * Every sphere centre that rodIntersection returns lies within its rod, but
+ * for two: S1, when the lines' intersection p lies inside rod 1 only, and S2,
+ * when it lies inside rod 2 only.  So where the centres are farther apart than
+ * both half lengths and the contact distance, a contact needs p inside rod 1
+ * and a point of rod 2 within the contact distance of line 1 (or the same with
+ * the rods exchanged).  With sa the distance of centre 1 from line 2, sb that
+ * of centre 2 from line 1 and n the sine of the angle between them, p is
+ * |sa / n| from centre 1 and |sb / n| from centre 2, and a rod's points come
+ * as near the other's line as |s| - h |n|.
+ *
+ * Both tolerances (2^-9 of the lengths, and 64 roundings of the coordinates)
+ * lie above the roundings of rodIntersection when |n| > 2^-7, whose quotients
+ * by n it bounds; rods nearer parallel are left to it.  A NaN is never apart. */
+template <typename T>
+CBM_HD bool cbm_rod_apart(const CbmRodGeom<T>& a, T d1, const CbmRodGeom<T>& b, T d2) {
+  const T eps = sizeof(T) == 8 ? (T)2.220446049250313e-16 : (T)1.1920929e-7f;
+  const T cx = a.x - b.x, cy = a.y - b.y;
+  const T h1 = fabs(a.l) * (T)0.5, h2 = fabs(b.l) * (T)0.5, D = (fabs(d1) + fabs(d2)) * (T)0.5;
+  const T S = h1 + h2 + D;
+  const T tol = (S + (fabs(cx) + fabs(cy))) * (T)0.001953125 +
+                (fabs(a.x) + fabs(a.y)) * ((T)64 * eps);
+  if (!(cx * cx + cy * cy > (S + tol) * (S + tol))) return false;
+  const T n = fabs(a.c * b.s - a.s * b.c);
+  const T sa = fabs(cx * b.s - cy * b.c), sb = fabs(cx * a.s - cy * a.c);
+  if (!(n > (T)0.0078125)) return false;
+  const T r1 = h1 * n, r2 = h2 * n;
+  return (sa > r1 + tol || sb > r2 + (D + tol)) && (sb > r2 + tol || sa > r1 + (D + tol));
+}
+
 #endif /* CBM_RODS_MATH_H */
