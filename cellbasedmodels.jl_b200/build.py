@@ -23,6 +23,7 @@ DEPS = SOURCES + [
     os.path.join(HERE, "csrc", "cbm_small.cuh"),
     os.path.join(HERE, "csrc", "cbm_stencil_vec.cuh"),
     os.path.join(HERE, "csrc", "cbm_tile.cuh"),
+    os.path.join(HERE, "csrc", "cbm_tile_filter.h"),
     os.path.join(HERE, "..", "include", "cbm_b200.h"),
     os.path.join(HERE, "..", "include", "cbm_rng.h"),
     os.path.join(HERE, "..", "include", "cbm_rods_math.h"),

@@ -498,6 +498,9 @@ void enqueue_step(cbm_adjoint* a, const AdjParams<T>& A, int* starts, int blocks
   }
   P.edge = A.edge;
   P.cut2 = A.cut2;
+  const double c = std::max(a->cfg.r_rep, a->cfg.r_att);
+  P.tile_scale = (T)tile_scale(c, a->cfg.cell_edge);
+  P.tile_cut = tile_cut(c, a->cfg.cell_edge);
   P.k_rep = A.k;
   P.r_rep = A.rho;
   P.k_att = A.a;

@@ -245,6 +245,8 @@ T exact_reciprocal(T v) {
   return (r > (T)0 && std::isfinite(r) && r * v == (T)1) ? r : (T)0;
 }
 
+double cutoff(const cbm_config& k) { return k.r_rep > k.r_att ? k.r_rep : k.r_att; }
+
 template <typename T>
 Params<T> params(const cbm_ctx* c, int parity) {
   using V4 = typename V4T<T>::type;
@@ -354,6 +356,8 @@ Params<T> params(const cbm_ctx* c, int parity) {
   P.skin2 = bound2<T>(k.skin);
   P.skin2_lo = bound2_lo<T>(k.skin);
   P.tiled = c->tile_blocks > 0;
+  P.tile_scale = (T)tile_scale(cutoff(k), k.cell_edge);
+  P.tile_cut = tile_cut(cutoff(k), k.cell_edge);
   P.force_in_list = (T)(k.r_rep > k.r_att ? k.r_rep : k.r_att) <= (T)k.skin ? 1 : 0;
   P.cut_reach = (T)((k.r_rep > k.r_att ? k.r_rep : k.r_att) * (1.0 + 1e-4));
   P.skin_reach = (T)(k.skin * (1.0 + 1e-4));
@@ -386,16 +390,14 @@ bool rule_needed(const cbm_config& k) {
 // the atomic rule path reads the committed field from a snapshot
 bool needs_snapshot(const cbm_config& k) { return k.uptake != 0 && exchanges(k) && !orders_exchange(k); }
 
-double cutoff(const cbm_config& k) { return k.r_rep > k.r_att ? k.r_rep : k.r_att; }
-
 // The 3D cell walks that k_agent_de_tile takes: of the committed positions
 // (no wall reflection and no stage positions, whose agents may lie outside
 // the cells they are filed in), with CellLinked, or with CLVD in the steps
-// with births or deaths.
+// with births or deaths, where the tile's filter serves (tile_scale).
 bool walk_by_tile(const cbm_config& k) {
   return k.dims == 3 && k.walls != CBM_WALLS_REFLECT &&
          (k.integrator == CBM_INT_EULER || k.integrator == CBM_INT_EM) &&
-         cutoff(k) <= kTileMaxCutoff &&
+         tile_scale(cutoff(k), k.cell_edge) != 0.0 &&
          (k.neighbors == CBM_NEIGH_CELL_LINKED ||
           (k.neighbors == CBM_NEIGH_CLVD && k.fate != CBM_FATE_NONE));
 }

@@ -143,6 +143,8 @@ struct Params {
   T skin2_lo;               // skin^2 times 1 - 1e-5, rounded down: below it d < skin for certain
   int force_in_list;        // (T)cutoff <= (T)skin: every pair with a force term is in the list
   T cut_reach, skin_reach;  // cutoff and skin times 1 + 1e-4: cell-pruning radii
+  T tile_scale;             // the tiled walk's filter (cbm_tile_filter.h): its unit of length
+  float tile_cut;           // and the cutoff in it
   T wall_force, wall_range, drift_linear;
   T v_div, div_sep, p_death;
   T dx_m[3];

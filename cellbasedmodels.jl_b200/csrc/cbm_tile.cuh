@@ -4,18 +4,19 @@
 // sit in one or a few cells of one row and share nearly all their candidates.
 // The filter (which candidates may lie within the cutoff) is a contraction:
 //     |xi - xj|^2 - R^2 = (|xi|^2 - R^2) + |xj|^2 - 2 xi . xj
-// over the coordinates relative to the tile, so 16 agents x 8 candidates are
-// one mma.m16n8k8 (half inputs, float accumulators), and the sign of an
+// over the coordinates relative to the tile, in units of the cutoff's power of
+// two (cbm_tile_filter.h), so 16 agents x 8 candidates are one mma.m16n8k8 (half inputs, float accumulators), and the sign of an
 // accumulator is the decision: one funnel shift per pair collects it into a
 // word of 32 decisions (against about eleven instructions per pair when a
 // thread tests its own candidates).  The filter only has to keep every pair
-// that the evaluation's exact test keeps (see tile_row); the evaluation then
+// that the evaluation's exact test keeps (tile_row); the evaluation then
 // walks each agent's own words in candidate order and computes the terms
 // exactly as the reference does, so the sums are unchanged, bit for bit.
 #pragma once
 #include <cuda_fp16.h>
 
 #include "cbm_kernels.cuh"
+#include "cbm_tile_filter.h"
 
 namespace cbm {
 
@@ -38,13 +39,6 @@ static_assert(kTileWords % 4 == 0 && kTileRefill % 4 == 0, "the filter takes fou
 // of 8 banks, so that the eight rows of an ldmatrix (two records of each of
 // four words) fall into different banks
 constexpr int kTileWordStride = 32 * 16 + 32;
-// Largest |coordinate| relative to the tile that the half records hold with
-// the bounds of tile_row; farther agents and candidates are always kept.
-constexpr float kTileReach = 100.f;
-// cutoffs above this keep the per-thread walk (R^2 must stay far below the
-// largest half)
-constexpr double kTileMaxCutoff = 50.0;
-
 template <typename S>
 __device__ __forceinline__ void tile_begin(S& s) {  // the empty word
   s.word[kTileWords * 32 + (threadIdx.x & 31)] = 0u;
@@ -83,56 +77,11 @@ __device__ __forceinline__ void mma_16x8x8(float* d, unsigned a0, unsigned a1, u
       : "r"(a0), "r"(a1), "r"(b), "f"(ca), "f"(cb));
 }
 
-// A candidate's record, half (x, y | z, nh | nl, 0 | 0, 0) with nh + nl its
-// squared norm: the k dimension of the contraction.  A candidate out of reach
-// (or not a number) is kept whatever the agent, one beyond its run never.
-__device__ __forceinline__ uint4 tile_candidate(float x, float y, float z, bool valid, bool* far) {
-  const float hx = __half2float(__float2half_rn(x));
-  const float hy = __half2float(__float2half_rn(y));
-  const float hz = __half2float(__float2half_rn(z));
-  const float n = __fmaf_rn(hz, hz, __fmaf_rn(hy, hy, hx * hx));
-  const float nh = __half2float(__float2half_rn(n));
-  uint4 r = make_uint4(half2_bits(hx, hy), half2_bits(hz, nh), half2_bits(n - nh, 0.f), 0u);
-  // (a NaN fails the test of n, whatever fmaxf makes of it)
-  if (!(fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z)) <= kTileReach) || !(n < 60000.f)) {
-    r = make_uint4(0u, half2_bits(0.f, -60000.f), 0u, 0u);
-    *far = true;
-  }
-  if (!valid) r = make_uint4(0u, half2_bits(0.f, 65504.f), 0u, 0u);
-  return r;
-}
-
-// An agent's row, half (-2x, -2y | -2z, 1 | 1, 0 | 0, 0), and the start of its
-// accumulator, |x|^2 - R^2.  With u = 2^-11 (half rounding) and X the agent's
-// largest |coordinate|, a candidate inside the cutoff c has coordinates of at
-// most X + c, so each component of the difference of the rounded positions is
-// within E = u (2X + c) (plus float rounding) of the exact one, and the
-// rounded distance is below R = c + sqrt(3) E.  The contraction adds at most
-// six products that are exact in float: its roundings, and those of nh + nl
-// and of R, stay below 2^-18 (|x| + R)^2 for every pair closer than R; the
-// start is lowered by 2^-16 of it.  Agents out of reach keep every candidate
-// of their runs, lanes outside the tile's row none.
-__device__ __forceinline__ uint4 tile_row(float x, float y, float z, float c, bool member,
-                                          float* start) {
-  const float X = fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z));
-  const float hx = __half2float(__float2half_rn(x));
-  const float hy = __half2float(__float2half_rn(y));
-  const float hz = __half2float(__float2half_rn(z));
-  const float n = __fmaf_rn(hz, hz, __fmaf_rn(hy, hy, hx * hx));
-  const float R = c + 1.7320509f * (4.886e-4f * (2.f * X + c) + 3e-6f);
-  const float m = sqrtf(n) + R;
-  *start = n - R * R - 1.52587890625e-5f * (m * m);
-  uint4 r = make_uint4(half2_bits(-2.f * hx, -2.f * hy), half2_bits(-2.f * hz, 1.f),
-                       half2_bits(1.f, 0.f), 0u);
-  if (!(X <= kTileReach)) {
-    r = make_uint4(0u, half2_bits(0.f, 1.f), half2_bits(1.f, 0.f), 0u);
-    *start = -61000.f;
-  }
-  if (!member) {
-    r = make_uint4(0u, 0u, 0u, 0u);
-    *start = 1.f;
-  }
-  return r;
+// The records of tile_candidate and tile_row as eight halves: k = 0 .. 7 of
+// the contraction.
+__device__ __forceinline__ uint4 tile_record(const TileRecord& r) {
+  return make_uint4(half2_bits(r.v[0], r.v[1]), half2_bits(r.v[2], r.v[3]),
+                    half2_bits(r.v[4], 0.f), 0u);
 }
 
 // The branch-free form's coefficients (cbm_pair.cuh) of the model.
@@ -261,7 +210,7 @@ __device__ __forceinline__ void tile_forces(const Params<T>& P, TileSmem& S, con
   // 76, the 256^3 medium's 159 against 55, the adjoint's 65536 agents at 0.13
   // per unit volume 195 against 115 us a step.)
   const int most = __reduce_max_sync(kFull, in ? cand : 0);
-  bool by_tile = 20 * most > 350 * n_rows && P.cut2 <= (T)(1.1 * kTileMaxCutoff * kTileMaxCutoff);
+  bool by_tile = 20 * most > 350 * n_rows && P.tile_scale != (T)0;
   if (by_tile) {
     int words = 0;
     for (unsigned l = leaders; l; l &= l - 1u)
@@ -339,12 +288,17 @@ __device__ __forceinline__ void tile_forces(const Params<T>& P, TileSmem& S, con
     return;
   }
 
-  const float c = sqrtf((float)P.cut2) * 1.000002f;
+  const float c = P.tile_cut;
+  // The filter's unit, a power of two: the fused operation that scales rounds
+  // as the difference alone does.  (A constant operand in Float32, where a
+  // register for it made the walk of 1e6 agents 2.056 ms instead of 2.037; a
+  // register in Float64, without which that of 1.5e5 took 255 us, not 245.)
+  std::conditional_t<sizeof(T) == 4, const T&, const T> scale = P.tile_scale;
   const int g = lane >> 2, q4 = lane & 3;
   const unsigned rec = (unsigned)__cvta_generic_to_shared(S.rec);
   unsigned row_a[4];       // A fragments: agents 0-7, 8-15, 16-23, 24-31
   float start[4];          // accumulator starts of agents g, g + 8, g + 16, g + 24
-  T org[3];
+  T org[3];  // minus the middle of the row's cells, in the filter's unit
   bool member = false;
   unsigned rem = leaders;
   int run = 9, k0 = 0, k1 = 0;   // next candidate and end of the run being queued
@@ -362,16 +316,16 @@ __device__ __forceinline__ void tile_forces(const Params<T>& P, TileSmem& S, con
         rem &= rem - 1u;
         member = (gm >> lane) & 1u;
         if (n_rows > 1) unite(gm);
-        // coordinates relative to the middle of the row's cells
         const int qa = __shfl_sync(kFull, q0, lead), qb = __shfl_sync(kFull, q0, 31 - __clz(gm));
-        org[0] = P.box_lo[0] + ((T)(qa + qb) * (T)0.5 - (T)0.5) * P.edge;
-        org[1] = P.box_lo[1] + ((T)__shfl_sync(kFull, q1, lead) - (T)0.5) * P.edge;
-        org[2] = P.box_lo[2] + ((T)__shfl_sync(kFull, q2, lead) - (T)0.5) * P.edge;
+        org[0] = -scale * (P.box_lo[0] + ((T)(qa + qb) * (T)0.5 - (T)0.5) * P.edge);
+        org[1] = -scale * (P.box_lo[1] + ((T)__shfl_sync(kFull, q1, lead) - (T)0.5) * P.edge);
+        org[2] = -scale * (P.box_lo[2] + ((T)__shfl_sync(kFull, q2, lead) - (T)0.5) * P.edge);
+        const T xs[3] = {fma(xi[0], scale, org[0]), fma(xi[1], scale, org[1]),
+                         fma(xi[2], scale, org[2])};
         float st;
-        far = far || !(fabs(xi[0] - org[0]) + fabs(xi[1] - org[1]) + fabs(xi[2] - org[2]) <= (T)kTileReach);
-        const uint4 a = tile_row((float)(xi[0] - org[0]), (float)(xi[1] - org[1]),
-                                 (float)(xi[2] - org[2]), c, member, &st);
-        *reinterpret_cast<uint4*>(S.rec + lane * 16) = a;
+        far = far || !(fabs(xs[0]) + fabs(xs[1]) + fabs(xs[2]) <= (T)kTileReach);
+        *reinterpret_cast<uint4*>(S.rec + lane * 16) =
+            tile_record(tile_row((float)xs[0], (float)xs[1], (float)xs[2], c, member, &st));
 #pragma unroll
         for (int k = 0; k < 4; ++k) start[k] = __shfl_sync(kFull, st, g + 8 * k);
         __syncwarp();
@@ -429,9 +383,9 @@ __device__ __forceinline__ void tile_forces(const Params<T>& P, TileSmem& S, con
         for (int j = 0; j < 4; ++j) {
           T xj[3];
           to3<T>(v[j], xj);
-          *reinterpret_cast<uint4*>(S.rec + j * kTileWordStride + lane * 16) =
-              tile_candidate((float)(xj[0] - org[0]), (float)(xj[1] - org[1]),
-                             (float)(xj[2] - org[2]), lane < (S.info[w + j] >> 8), &far);
+          *reinterpret_cast<uint4*>(S.rec + j * kTileWordStride + lane * 16) = tile_record(
+              tile_candidate((float)fma(xj[0], scale, org[0]), (float)fma(xj[1], scale, org[1]),
+                             (float)fma(xj[2], scale, org[2]), lane < (S.info[w + j] >> 8), &far));
         }
         __syncwarp();
         const int wn = w + 4 == kTileWords ? 0 : w + 4;
