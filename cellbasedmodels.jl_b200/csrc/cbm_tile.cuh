@@ -172,7 +172,7 @@ __device__ __forceinline__ void tile_forces(const Params<T>& P, TileSmem& S, con
     const int py = q1 + r % 3 - 1, pz = q2 + r / 3 - 1;
     lo[r] = hi[r] = 0;
     if (py >= 0 && py < ny && pz >= 0 && pz < nz) {
-      const int row = row0 + nx * (r % 3 + ny * (r / 3));
+      const int row = tile_run_row(row0, nx, ny, r);
       lo[r] = ld(P.cell_start + row + xa);
       hi[r] = ld(P.cell_start + row + xb + 1);
     }
@@ -349,7 +349,7 @@ __device__ __forceinline__ void tile_forces(const Params<T>& P, TileSmem& S, con
           int w = pos + k;
           w = w >= kTileWords ? w - kTileWords : w;
           S.base[w] = b;
-          S.info[w] = (unsigned short)(run | ((k1 - b < 32 ? k1 - b : 32) << 8));
+          S.info[w] = tile_info(run, k1 - b < 32 ? k1 - b : 32);
         }
         n += take;
         pos += take;
@@ -363,7 +363,7 @@ __device__ __forceinline__ void tile_forces(const Params<T>& P, TileSmem& S, con
       }
       for (; n & 3; ++n) {  // whole groups of four
         S.base[pos] = 0;
-        S.info[pos] = 0;
+        S.info[pos] = kTilePad;
         ++pos;
       }
       __syncwarp();
@@ -420,7 +420,7 @@ __device__ __forceinline__ void tile_forces(const Params<T>& P, TileSmem& S, con
             const int r = S.info[w + j] & 255, b = S.base[w + j];
             if (r != cur) {
               cur = r;
-              const int row = row0 + nx * (r % 3 + ny * (r / 3));
+              const int row = tile_run_row(row0, nx, ny, r);
               rlo = ld(P.cell_start + row + xa);
               rhi = ld(P.cell_start + row + xb + 1);
             }

@@ -50,6 +50,22 @@ CBM_FILTER_HD float half_round(float v) {
 #endif
 }
 
+// Runs r = 0 .. 8 of a walk are the rows of cells (dy, dz) = (r % 3 - 1,
+// r / 3 - 1) around an agent's own.  First cell of the row of run r; row0: of
+// run 0, which is negative for agents in the grid's first layers (those below
+// the box, or with a NaN coordinate), where the rows outside the grid have no
+// run.
+CBM_FILTER_HD int tile_run_row(int row0, int nx, int ny, int r) {
+  return row0 + nx * (r % 3 + ny * (r / 3));
+}
+// What the queue notes of a word: its run and its candidates.
+CBM_FILTER_HD unsigned short tile_info(int run, int candidates) {
+  return (unsigned short)(run | (candidates << 8));
+}
+// An empty word that fills a group of four.  Its agents look its run up too:
+// their own row, which every grid has.
+constexpr unsigned short kTilePad = 4;
+
 struct TileRecord {
   float v[5];  // stored as halves
 };

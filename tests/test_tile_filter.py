@@ -1,7 +1,7 @@
 """The tiled force walk's candidate filter against the pair test itself, on the
 CPU: every pair with a force must be kept, whatever the unit of length, with
 the stated bound of the contraction's roundings held against it, and few
-others may be."""
+others may be.  And the cells that a word's agents look up, which must exist."""
 import os
 import subprocess
 
@@ -116,13 +116,55 @@ int main() {
 }
 """
 
+# The masks of words shared by agents of several cells read cell_start at the
+# first cell and one past the last of the word's run, for every word that the
+# queue writes: those of the rows that the grid has, and the filling of a
+# group of four.  Agents sit in every cell, the outermost layers included.
+ROWS = r"""
+#include <cstdio>
+#include "cbm_tile_filter.h"
+using namespace cbm;
+int main() {
+  int bad = 0;
+  for (int nx = 1; nx <= 4; ++nx)
+    for (int ny = 1; ny <= 4; ++ny)
+      for (int nz = 1; nz <= 4; ++nz)
+        for (int c = 0; c < nx * ny * nz; ++c) {
+          const int q0 = c % nx, q1 = (c / nx) % ny, q2 = c / (nx * ny);
+          const int row0 = nx * (q1 - 1 + ny * (q2 - 1));
+          const int xa = q0 > 0 ? q0 - 1 : 0, xb = q0 < nx - 1 ? q0 + 1 : nx - 1;
+          auto look = [&](unsigned short info) {
+            const int row = tile_run_row(row0, nx, ny, info & 255);
+            if (row + xa < 0 || row + xb + 1 > nx * ny * nz) {
+              if (!bad) std::printf("grid %d %d %d cell %d run %d: row %d\n", nx, ny, nz, c, info & 255, row);
+              bad = 1;
+            }
+          };
+          for (int r = 0; r < 9; ++r) {
+            const int py = q1 + r % 3 - 1, pz = q2 + r / 3 - 1;
+            if (py >= 0 && py < ny && pz >= 0 && pz < nz) look(tile_info(r, 32));
+          }
+          look(kTilePad);
+        }
+  return bad | (kTilePad >> 8);
+}
+"""
 
-def test_filter_keeps_every_partner(tmp_path):
+
+def run_program(tmp_path, source):
     src = tmp_path / "filter.cpp"
-    src.write_text(PROGRAM)
+    src.write_text(source)
     exe = tmp_path / "filter"
     subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-I",
                     os.path.join(ROOT, "cellbasedmodels.jl_b200", "csrc"), str(src), "-o",
                     str(exe)], check=True)
     out = subprocess.run([str(exe)], capture_output=True, text=True)
     assert out.returncode == 0, out.stdout
+
+
+def test_filter_keeps_every_partner(tmp_path):
+    run_program(tmp_path, PROGRAM)
+
+
+def test_words_look_up_existing_cells(tmp_path):
+    run_program(tmp_path, ROWS)
