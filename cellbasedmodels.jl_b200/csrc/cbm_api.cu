@@ -87,11 +87,13 @@ struct cbm_ctx {
   void* c[2] = {};
   void* grad[2][3] = {};
   int* gather_box = nullptr;  // cell-box tables of the exchange's gather (k_gather_box)
-  // exchange by lists: buckets' first entries, entries, Float64 weights
+  // exchange by lists: buckets' first entries, entries, Float64 weights, and
+  // room to sort the entries of crowded nodes
   unsigned* link_head = nullptr;
   unsigned link_buckets = 0;
   uint4* link = nullptr;
   void* link_w = nullptr;
+  unsigned long long* link_sort = nullptr;
   Counters* ctr = nullptr;
   Counters* h_ctr = nullptr;   // pinned staging of the counters an upload writes
   int* scratch_int = nullptr;  // n_max ints for inspection calls
@@ -295,6 +297,7 @@ Params<T> params(const cbm_ctx* c, int parity) {
   for (unsigned b = c->link_buckets; b > 1; b >>= 1) --P.link_shift;
   P.link = c->link;
   P.link_w = (T*)c->link_w;
+  P.link_sort = c->link_sort;
   P.scan_state = c->scan_state;
   P.nbr_n = c->nbr_n;
   P.nbr_list = c->nbr_list;
@@ -477,9 +480,13 @@ void enqueue_medium_rule(cbm_ctx* c, const Params<T>& P) {
   }
 }
 
+// the heads and the count that follows them, to a length that clears by
+// whole vectors
+size_t link_head_bytes(const cbm_ctx* c) { return ((size_t)c->link_buckets + 64) * 4; }
+
 template <typename T, int D>
 void enqueue_links(cbm_ctx* c, const Params<T>& P) {
-  cudaMemsetAsync(c->link_head, 0xff, (size_t)c->link_buckets * 4, c->stream);
+  cudaMemsetAsync(c->link_head, 0xff, link_head_bytes(c), c->stream);
   PROF("k_medium_links");
   k_medium_links<T, D><<<grid_blocks(c->cfg.n_max << D), kTile, 0, c->stream>>>(P);
 }
@@ -1160,9 +1167,10 @@ int cbm_create(cbm_ctx** out, const cbm_config* cfg) {
     if (orders_exchange(k) && ne * kListNodes <= (unsigned long long)c->n_nodes) {
       c->link_buckets = 1024;
       while (c->link_buckets < ne) c->link_buckets *= 2;
-      c->link_head = (unsigned*)dalloc(c, (size_t)c->link_buckets * 4, &ok);
+      c->link_head = (unsigned*)dalloc(c, link_head_bytes(c), &ok);
       c->link = (uint4*)dalloc(c, ne * sizeof(uint4), &ok);
       if (S == 8) c->link_w = dalloc(c, ne * S, &ok);
+      c->link_sort = (unsigned long long*)dalloc(c, ne * 8, &ok);
     }
   }
   c->ctr = (Counters*)dalloc(c, sizeof(Counters), &ok);

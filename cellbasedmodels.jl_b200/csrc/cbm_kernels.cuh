@@ -89,11 +89,13 @@ struct Params {
   int* cell_start;      // n_cells + 1
   const int* gather_box;  // per medium axis d, per node q: gather_cell_lo, then gather_cell_hi
   // entries (agent, stencil node) of the exchange by lists: entry s * 2^D + k
-  unsigned* link_head;  // first entry of each bucket, kNoLink for none
+  unsigned* link_head;  // first entry of each bucket, kNoLink for none; then the used part of
+                        // link_sort, less one
   unsigned link_mask;   // buckets less one (a power of two)
   int link_shift;       // 35 less their logarithm
   uint4* link;          // next entry of the bucket, node, agent, weight (Float32)
   T* link_w;            // weights (Float64)
+  unsigned long long* link_sort;  // crowded nodes' entries: as many in all as there are entries
   unsigned long long* scan_state;
   // Verlet list in slot space: entry k of the row of slot s at k * n_max + s
   int* nbr_n;
@@ -851,52 +853,205 @@ __global__ void __launch_bounds__(kTile) k_medium_links(Params<T> P) {
   P.link[e] = make_uint4(next, node, (unsigned)P.IA[s], bits);
 }
 
+// keys[0, m) in ascending order, by one block: a bitonic network in which
+// every comparison puts the smaller key first, so that the keys it would have
+// beyond m never move below m and are left out.  Four pairs a thread in flight.
+static __device__ __noinline__ void sort_by_block(unsigned long long* keys, int m) {
+  constexpr int U = 4;
+  for (int k = 2; (k >> 1) < m; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      const bool flip = j == k >> 1;  // pair i of a run of 2 j with its mirror image
+      const int pairs = (m + 2 * j - 1) / (2 * j) * j;
+      for (int t0 = threadIdx.x; t0 < pairs; t0 += kTile * U) {
+        unsigned long long x[U], y[U];
+        int lo[U], hi[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int t = t0 + kTile * u, at = t & (j - 1);
+          lo[u] = 2 * (t - at) + at;
+          hi[u] = flip ? 2 * (t - at) + 2 * j - 1 - at : lo[u] + j;
+          if (t >= pairs) hi[u] = m;
+          x[u] = y[u] = 0ull;
+          if (hi[u] < m) {
+            x[u] = keys[lo[u]];
+            y[u] = keys[hi[u]];
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (x[u] > y[u]) {
+            keys[lo[u]] = y[u];
+            keys[hi[u]] = x[u];
+          }
+      }
+      __syncthreads();
+    }
+}
+
+// What k_medium_apply leaves to a block, besides a node's number of entries:
+// nodes with lists too long to walk, ...
+constexpr int kSearch = 0;
+constexpr int kSearchFirst = -1;  // ... even to tell whether the entry is its node's first
+
+// The node of entry e, summed by one block: its entries are put, key above
+// number, into a stretch of `sorted` (`used`: its used part, less one), sorted
+// and added in order.  m > 0: the node has m entries, of which e is the first
+// in its list.  With a longer list, or fewer than 1024 m entries in `total`,
+// they are searched for among all (a walk is one read after another, about 300
+// cycles, the search about 0.3 cycles an entry), and come in slot order, which
+// is the keys' when the agents are in one cell; in doubt the entry of the
+// lowest number sums.  Not inlined, so that nothing of it takes registers from
+// the nodes with a few entries.
+template <typename T>
+__device__ __noinline__ void crowded_node(const uint4* link, const T* link_w,
+                                          unsigned long long* sorted, unsigned* used, T* c,
+                                          unsigned e, int m, unsigned total, unsigned K, T amt,
+                                          T uptake) {
+  constexpr int W = kTile / 32, U = 4;
+  __shared__ unsigned s_at;
+  __shared__ int s_count[W];
+  __shared__ T s_term[2][kTile];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const unsigned node = link[e].y;
+  auto key = [&](unsigned f) {
+    return ((unsigned long long)(link[f].z * K + f % K) << 32) | f;
+  };
+  if (m > 0 && total >> 10 >= (unsigned)m) {
+    if (threadIdx.x == 0) {
+      s_at = atomicAdd(used, (unsigned)m) + 1u;
+      unsigned at = s_at;
+      for (unsigned f = e; f != kNoLink;) {
+        const uint4 q = link[f];
+        if (q.y == node) sorted[at++] = key(f);
+        f = q.x;
+      }
+    }
+    __syncthreads();
+  } else {
+    const unsigned part = (total + kTile - 1) / kTile * 32;  // entries of a warp
+    const unsigned a = w * part, b = a + part < total ? a + part : total;
+    int count = 0;
+    bool earlier = false;
+    for (unsigned f0 = a + lane; f0 < b; f0 += 32 * U) {
+      unsigned y[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) y[u] = f0 + 32 * u < b ? link[f0 + 32 * u].y : ~node;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        count += y[u] == node;
+        earlier = earlier || (y[u] == node && f0 + 32 * u < e);
+      }
+    }
+    count = __reduce_add_sync(kFull, count);
+    if (lane == 0) s_count[w] = count;
+    if (__syncthreads_or(m == kSearchFirst && earlier)) return;
+    int at = 0;
+    m = 0;
+    for (int v = 0; v < W; ++v) {
+      at += v < w ? s_count[v] : 0;
+      m += s_count[v];
+    }
+    if (threadIdx.x == 0) s_at = atomicAdd(used, (unsigned)m) + 1u;
+    __syncthreads();
+    unsigned long long* const keys = sorted + s_at;
+    for (unsigned f0 = a; f0 < b; f0 += 32) {
+      const unsigned f = f0 + lane;
+      const bool hit = f < b && link[f].y == node;
+      const unsigned hits = __ballot_sync(kFull, hit);
+      if (hit) keys[at + __popc(hits & ((1u << lane) - 1u))] = key(f);
+      at += __popc(hits);
+    }
+    __syncthreads();
+  }
+  unsigned long long* const keys = sorted + s_at;
+  bool unsorted = false;
+  for (int i = threadIdx.x; i < m - 1; i += kTile) unsorted = unsorted || keys[i] > keys[i + 1];
+  if (__syncthreads_or(unsorted)) sort_by_block(keys, m);
+  // one thread adds the terms of a stretch while the others make the next's
+  T acc = c[node];
+  const T net = uptake != (T)0 ? amt - uptake * acc : amt;
+  for (int base = 0, n = 0; base < m + kTile; base += kTile) {
+    T* const term = s_term[(base / kTile) & 1];
+    const int i = base + threadIdx.x;
+    if (i < m) {
+      const unsigned f = (unsigned)keys[i];
+      if constexpr (sizeof(T) == 4) term[threadIdx.x] = __uint_as_float(link[f].w) * net;
+      else term[threadIdx.x] = link_w[f] * net;
+    }
+    if (threadIdx.x == 0) {
+      const T* const before = s_term[((base / kTile) & 1) ^ 1];
+#pragma unroll 16
+      for (int u = 0; u < n; ++u) acc = acc + before[u];
+    }
+    n = m - base < kTile ? m - base : kTile;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) c[node] = acc;
+}
+
 // One thread an entry; the first of its node's entries in the bucket's list
 // sums them.  Up to kOrder entries are ordered in registers; more take as
-// many passes, each over the kOrder smallest keys above the last pass's.
+// many passes, each over the kOrder smallest keys from the last pass's on.
+// That is m^2 / 4 dependent reads for m entries, so a node with more than
+// kCrowd, or a list of more than kLongest, is left to the block (crowded_node):
+// agents that gather on a node, or past the field's border, whose node then
+// has 2^D entries of each.  Eight neighboring nodes with m entries each, 3D
+// Float32: 85 us for m = 64 by passes, 137 for 65, 276 for 500 and 1170 for
+// 4000 by the block (by the gather k_secrete_rows: 285 for 60, 1590 for 500,
+// 15100 for 4000).  Seven blocks an SM (36 registers): with eight as with six
+// the step of 2e5 agents on 256^3 nodes is slower (175.3 us).
 template <typename T, int D>
-__global__ void __launch_bounds__(kTile) k_medium_apply(Params<T> P) {
-  constexpr int K = 1 << D;
-  constexpr int kOrder = 4;
+__global__ void __launch_bounds__(kTile, sizeof(T) == 4 ? 7 : 6) k_medium_apply(Params<T> P) {
+  constexpr unsigned K = 1 << D;
+  constexpr int kOrder = 4, kCrowd = 64, kLongest = 1024;
+  constexpr unsigned kNone = 0xffffffffu;  // above every key (agent * K + stencil node)
+  __shared__ int s_crowd[kTile];           // as crowded_node takes it
+  __shared__ unsigned s_mask[kTile / 32];
   const unsigned e = blockIdx.x * kTile + threadIdx.x;
-  if (e >= (unsigned)P.ctr->N[P.parity] * K) return;
-  const uint4 own = P.link[e];
-  const unsigned node = own.y;
-  T acc = P.c_cur[node];
-  for (unsigned f = P.link_head[link_bucket(P, node)]; f != e;) {
-    const uint4 m = P.link[f];
-    if (m.y == node) return;
-    f = m.x;
-  }
-  auto weight = [&](unsigned f, const uint4& m) -> T {
-    if constexpr (sizeof(T) == 4) return __uint_as_float(m.w);
-    else return P.link_w[f];
-  };
-  const T amt = P.secretion_amt;
-  // secretion less first-order uptake, at the committed value
-  const T net = P.uptake_amt != (T)0 ? amt - P.uptake_amt * acc : amt;
-  const long long kNone = 0x7fffffffffffffffll;
-  long long last = -1;
-  while (true) {
-    long long key[kOrder];
-    T w[kOrder];
-#pragma unroll
-    for (int q = 0; q < kOrder; ++q) {
-      key[q] = kNone;
-      w[q] = (T)0;
+  const unsigned total = (unsigned)P.ctr->N[P.parity] * K;
+  bool crowd = false;
+  if (e < total) {
+    const uint4 own = P.link[e];
+    const unsigned node = own.y;
+    T acc = P.c_cur[node];
+    bool first = true;
+    int steps = 0;
+    for (unsigned f = P.link_head[link_bucket(P, node)]; first && f != e;) {
+      const uint4 m = P.link[f];
+      first = m.y != node;
+      f = m.x;
+      if (++steps > kLongest && first) {  // (f == e too: every entry stops at the same place)
+        crowd = true;
+        s_crowd[threadIdx.x] = kSearchFirst;
+        first = false;
+      }
     }
-    int left = 0;  // entries above `last`
-    uint4 m = own;
-    for (unsigned f = e;;) {
-      if (m.y == node) {
-        long long kf = (long long)m.z * K + f % K;
-        T wf = weight(f, m);
-        if (kf > last) {
+    const T amt = P.secretion_amt;
+    // secretion less first-order uptake, at the committed value
+    const T net = P.uptake_amt != (T)0 ? amt - P.uptake_amt * acc : amt;
+    unsigned from = 0u;
+    while (first) {
+      unsigned key[kOrder];
+      T w[kOrder];
+#pragma unroll
+      for (int q = 0; q < kOrder; ++q) {
+        key[q] = kNone;
+        w[q] = (T)0;
+      }
+      int left = 0;  // entries with keys of at least `from`
+      steps = 0;
+      uint4 m = own;
+      for (unsigned f = e;;) {
+        unsigned kf = m.z * K + f % K;
+        if (m.y == node && kf >= from) {
+          T wf;
+          if constexpr (sizeof(T) == 4) wf = __uint_as_float(m.w);
+          else wf = P.link_w[f];
           ++left;
 #pragma unroll
           for (int q = 0; q < kOrder; ++q) {
             const bool before = kf < key[q];
-            const long long kt = before ? key[q] : kf;
+            const unsigned kt = before ? key[q] : kf;
             const T wt = before ? w[q] : wf;
             key[q] = before ? kf : key[q];
             w[q] = before ? wf : w[q];
@@ -904,18 +1059,34 @@ __global__ void __launch_bounds__(kTile) k_medium_apply(Params<T> P) {
             wf = wt;
           }
         }
+        f = m.x;
+        if (f == kNoLink || ++steps > kLongest) break;
+        m = P.link[f];
       }
-      f = m.x;
-      if (f == kNoLink) break;
-      m = P.link[f];
-    }
+      if (left > kCrowd || steps > kLongest) {
+        crowd = true;
+        s_crowd[threadIdx.x] = steps > kLongest ? kSearch : left;
+        first = false;
+        break;
+      }
 #pragma unroll
-    for (int q = 0; q < kOrder; ++q)
-      if (key[q] != kNone) acc = acc + w[q] * net;
-    if (left <= kOrder) break;
-    last = key[kOrder - 1];
+      for (int q = 0; q < kOrder; ++q)
+        if (key[q] != kNone) acc = acc + w[q] * net;
+      if (left <= kOrder) break;
+      from = key[kOrder - 1] + 1u;
+    }
+    if (first) P.c_cur[node] = acc;
   }
-  P.c_cur[node] = acc;
+  const unsigned mask = __ballot_sync(kFull, crowd);
+  if ((threadIdx.x & 31) == 0) s_mask[threadIdx.x >> 5] = mask;
+  if (!__syncthreads_or(crowd)) return;
+  for (int w = 0; w < kTile / 32; ++w)
+    for (unsigned todo = s_mask[w]; todo; todo &= todo - 1u) {
+      const int t = 32 * w + __ffs(todo) - 1;
+      crowded_node<T>(P.link, P.link_w, P.link_sort, P.link_head + P.link_mask + 1u, P.c_cur,
+                      blockIdx.x * kTile + t, s_crowd[t], total, K, P.secretion_amt, P.uptake_amt);
+      __syncthreads();
+    }
 }
 
 // ---------------------------------------------------------------------------
