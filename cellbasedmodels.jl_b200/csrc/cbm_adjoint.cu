@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(kTile) k_adj_backward(AdjParams<T> A) {
       const typename AV4<T>::type lo = A.lam[AV4<T>::dec(o.w)];
       T r[3];
       const T s2 = adj_diff(xi, o, r);
-      const bool mid = A.mid && s2 > (T)1e-12;
+      const bool mid = A.mid && s2 > (T)1e-12 && mid_root(s2);
       T inv0 = (T)0;
       const T dd = adj_sqrt(mid, s2, &inv0);  // every recorded pair has dd < r_att
       const bool rep = dd < A.rho;

@@ -135,12 +135,31 @@ __device__ __forceinline__ int floordiv(float a, float b) {
 // keeps one pair's operations in series with the next's).  Both refine the
 // hardware's approximation with fused operations and end in Markstein's
 // correction step (P. Markstein, "Computation of elementary functions on the
-// IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990): with h within
-// an ulp of 1 / (2 sqrt(x)) and g of sqrt(x), g + h (x - g^2) is the rounded
-// root; with y the rounded reciprocal of b and q within an ulp of a / b,
-// q + y (a - b q) is the rounded quotient.  Against the general functions:
-// Float32 equal on every significand at both exponent parities (the root, and
-// the reciprocal of every divisor), Float64 equal on 4e10 random operands.
+// IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990): with h near
+// 1 / (2 sqrt(x)) and g near sqrt(x), g + h (x - g^2) is the rounded root;
+// with y the rounded reciprocal of b and q near a / b, q + y (a - b q) is the
+// rounded quotient.
+//
+// They give the bits of the general operations.  Float32: every root of the
+// range and the reciprocal of every divisor are compared.  Float64, with
+// u = 2^-53 and an approximation good to 2^-18 (it is to 2^-20):
+//  - Of the first iteration's errors, g and h share all but three roundings,
+//    and the second halves what differs: both end within 2.5 u, and the last
+//    step within 12 u^2 of the root before it rounds.  The result can be wrong
+//    only if a midpoint of two numbers lies in between; there are 37 such x in
+//    [1, 4), and these are compared at every exponent.
+//  - inv is within 3.5 u of 1 / b, so y is 1 / b less at most (3.5 u)^2 of it,
+//    rounded: the rounded reciprocal unless a midpoint lies in between, at
+//    k u^2 / 2 from 1 / b with a whole k <= 12.  The quotient needs no more
+//    than |b y - 1| b < 2 u (1 - u) for b in [1, 2), since a - b m is a
+//    multiple of u times the spacing for every midpoint m; a y that is not the
+//    rounded one keeps to that too, unless b >= 2 - 12 u.  There the k of the
+//    number 2 - 2 n u is n^2 for odd n (for even n no midpoint is near), and
+//    errors are below 2.5 u, which leaves n = 1, the significand of ones: its y
+//    may be the power of two, and the quotient of a power of two then ends in
+//    a tie.  mid_root keeps the x with that root from here.  Also, q may be off
+//    by more than one place for both a and b among the last numbers of their
+//    binades, and these are compared.
 __device__ __forceinline__ float sqrt_mid(float x) {
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -179,10 +198,21 @@ __device__ __forceinline__ double sqrt_mid(double x, double* inv) {
   *inv = h + h;
   return __fma_rn(__fma_rn(-g, g, x), h, g);
 }
+// y: of sqrt_mid, whose root b is, for an x that mid_root takes
 __device__ __forceinline__ double div_mid(double a, double b, double y) {
   y = __fma_rn(__fma_rn(-b, y, 1.0), y, y);
   const double q = a * y;
   return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+
+// Whether div_mid takes the root of x as a divisor: a root of ones has an x of
+// 4^k (4 - 2^-50) or 4^k (4 - 2^-51).  (One comparison of the low word, which
+// a few other x fail: the Float64 walk of 1.5e5 agents takes 248 us with it,
+// 245 without.  Setting the bit of y instead: 248, and 3 % in communities of a
+// few hundred, which lose nothing so.)
+__device__ __forceinline__ bool mid_root(float) { return true; }
+__device__ __forceinline__ bool mid_root(double x) {
+  return (unsigned)__double2loint(x) < 0xfffffffeu;
 }
 
 // cellPos, src/neighbors.jl:636-638, 0-based; a NaN coordinate goes to the

@@ -165,7 +165,7 @@ __device__ __forceinline__ void small_de(const Params<T>& P, const PairLine<T>& 
       T sc = (T)0;
       if (q != s) {
         T inv = (T)0;
-        const bool mid = line.mid && s2 > (T)1e-12 && s2 < (T)1e12;
+        const bool mid = line.mid && s2 > (T)1e-12 && s2 < (T)1e12 && mid_root(s2);
         const T d = mid ? sqrt_mid(s2, &inv) : sqrt(s2);
         const bool rep = d < -line.nrrep;
         const T F = (rep ? line.krep : line.katt) * ((rep ? line.rrep : line.abase) - d);

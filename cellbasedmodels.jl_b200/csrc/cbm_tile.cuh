@@ -115,7 +115,8 @@ __device__ __forceinline__ int pair_terms4(const PairCoef<T>& c, const PairLine<
       const double d2 = pair_diff<double, 3>(xi, xj, e[u]);
       n2[u] = qq[u] == s ? -L.nfar2 : d2;
     }
-    if (plain && fmin(fmin(n2[0], n2[1]), fmin(n2[2], n2[3])) > 1e-12) {
+    if (plain && fmin(fmin(n2[0], n2[1]), fmin(n2[2], n2[3])) > 1e-12 && mid_root(n2[0]) &&
+        mid_root(n2[1]) && mid_root(n2[2]) && mid_root(n2[3])) {
       double sc[4];
       int in = 0;
 #pragma unroll
