@@ -548,7 +548,7 @@ int make_plan(cbm_adjoint* a, Plan& P, int n, int nsteps, int K, bool backward) 
   int* starts = (int*)get((size_t)(a->n_cells + 1) * 4);
   V4* xs = (V4*)get(nv * Kb);
   int* pair_n = backward ? (int*)get(n1 * 4 * Kb) : nullptr;
-  int* pair_list = (int*)get(n1 * 4 * (size_t)a->cap * Kb);
+  int* pair_list = backward ? (int*)get(n1 * 4 * (size_t)a->cap * Kb) : nullptr;
   P.gpart = (double*)get((size_t)step_blocks * 3 * 8);
   P.lpart = (double*)get((size_t)blocks * 8);
   if (!ok) {
@@ -564,7 +564,7 @@ int make_plan(cbm_adjoint* a, Plan& P, int n, int nsteps, int K, bool backward) 
   cudaStream_t st = a->stream;
   cudaGraph_t g = nullptr;
   // a step from cur to nxt; kept (slot positions and pairs) in place m of the
-  // segment, or, m < 0, in place 0 without its pair counts
+  // segment, or, m < 0, its positions in place 0 and no pairs
   auto step = [&](const V4* cur, V4* nxt, int m, bool file) {
     AdjParams<T> A = adj_params<T>(a, n);
     const size_t at = (size_t)(m < 0 ? 0 : m) * n1;
@@ -573,7 +573,7 @@ int make_plan(cbm_adjoint* a, Plan& P, int n, int nsteps, int K, bool backward) 
     A.xs = xs + at;
     A.cell_start = starts;
     A.pair_n = m < 0 ? nullptr : pair_n + at;
-    A.pair_list = pair_list + at * (size_t)a->cap;
+    A.pair_list = m < 0 ? nullptr : pair_list + at * (size_t)a->cap;
     A.file = file;
     enqueue_step<T>(a, A, starts, blocks);
   };
