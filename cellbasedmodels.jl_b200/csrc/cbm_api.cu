@@ -104,7 +104,8 @@ struct cbm_ctx {
   int n_sm = 148;             // multiprocessors of the device (grid of the compaction)
   int de_blocks = 1;          // persistent grid of the force kernel
   int tile_blocks = 0;        // resident blocks of k_agent_de_tile (0: not used)
-  void* pair_list = nullptr;  // its partner lists (cell walks only)
+  bool sparse = false;        // the walks that the tiles could take are made by threads
+  void* pair_list = nullptr;  // partner lists of the walks by threads
   void* pos32 = nullptr;      // Float64 3D cell walks: positions rounded to Float32
   void* pos_rows = nullptr;   // Float32 3D cell walks: positions as rows x | y | z
   int rows_stride = 0;
@@ -301,10 +302,11 @@ Params<T> params(const cbm_ctx* c, int parity) {
   P.scan_state = c->scan_state;
   P.nbr_n = c->nbr_n;
   P.nbr_list = c->nbr_list;
-  P.pair_list = (int4*)c->pair_list;
+  P.tiled = c->tile_blocks > 0 && !c->sparse;
+  P.pair_list = P.tiled ? nullptr : (int4*)c->pair_list;
   P.pair_cap4 = kPairCap4;
-  P.PA32 = (float4*)c->pos32;
-  P.PS = (float*)c->pos_rows;
+  P.PA32 = P.tiled ? nullptr : (float4*)c->pos32;
+  P.PS = P.tiled ? nullptr : (float*)c->pos_rows;
   P.ps_stride = c->rows_stride;
   P.c_cur = (T*)c->c[p];
   P.c_nxt = (T*)c->c[q];
@@ -358,7 +360,6 @@ Params<T> params(const cbm_ctx* c, int parity) {
   P.cut2 = bound2<T>(k.r_rep > k.r_att ? k.r_rep : k.r_att);
   P.skin2 = bound2<T>(k.skin);
   P.skin2_lo = bound2_lo<T>(k.skin);
-  P.tiled = c->tile_blocks > 0;
   P.tile_scale = (T)tile_scale(cutoff(k), k.cell_edge);
   P.tile_cut = tile_cut(cutoff(k), k.cell_edge);
   P.force_in_list = (T)(k.r_rep > k.r_att ? k.r_rep : k.r_att) <= (T)k.skin ? 1 : 0;
@@ -409,6 +410,28 @@ bool walk_by_thread(const cbm_config& k) {
   return k.dims == 3 && !walk_by_tile(k) &&
          (k.neighbors == CBM_NEIGH_CELL_LINKED ||
           (k.neighbors == CBM_NEIGH_CLVD && k.fate != CBM_FATE_NONE));
+}
+
+// Sparse communities of many agents are walked by threads: their tiles find
+// too few partners to share, and each lane's own candidates then wait on
+// gathers with thirteen warps an SM, in Float64 on 32-byte positions that
+// saturate L1 (82 %).  The walk by threads has full occupancy and, in Float64,
+// the filter's Float32 copy.  The measure is the mean number of agents in an
+// agent's cell, itself included.  Step in us, by tiles / by threads, cells of
+// 1.1 cutoffs:
+//   Float64, 1e6 agents     2.4 a cell 465 / 314   6.4: 506 / 412   8.2: 526 / 469   10: 564 / 574
+//            1e5            1.2: 50 / 45   3.2: 91 / 55   8.2: 92 / 73   10: 94 / 85   15: 114 / 110
+//            5e4            1.2: 33 / 40   3.2: 55 / 49   8.2: 65 / 62   10: 62 / 69
+//   Float32, 1e6            1.7: 201 / 230   3.2: 291 / 275   4.6: 364 / 295   8.2: 361 / 358   10: 385 / 435
+//            1e5            1.7: 42 / 46   3.2: 58 / 54   4.6: 63 / 55   8.2: 69 / 64   12: 78 / 77
+//            5e4            3.2: 40 / 48   4.6: 46 / 50
+constexpr long long kSparseFrom = 65536;
+bool may_be_sparse(const cbm_config& k) { return walk_by_tile(k) && k.n_max >= kSparseFrom; }
+// `now`: a margin keeps a community at the line where it is.
+bool is_sparse(const cbm_config& k, double per_cell, long long n, bool now) {
+  const double lo = k.precision == CBM_F64 ? 0.0 : 2.5, hi = k.precision == CBM_F64 ? 9.5 : 8.2;
+  const double m = now ? 1.1 : 1.0;
+  return n >= kSparseFrom && per_cell * m > lo && per_cell < hi * m;
 }
 
 // blocks of the 2D shared-memory stencils (one tile per block)
@@ -538,11 +561,11 @@ template <typename T, int D>
 void enqueue_agent_de(cbm_ctx* c, const Params<T>& P) {
   const unsigned grid = kPartnerLists<D> ? c->de_blocks : c->n_blocks;
   const int integ = c->cfg.integrator;
-  if (c->pos32) {
+  if (P.PA32) {
     PROF("k_pos32");
     k_pos32<T><<<c->n_blocks, kTile, 0, c->stream>>>(P);
   }
-  if (c->pos_rows) {
+  if (P.PS) {
     PROF("k_pos_rows");
     k_pos_rows<T><<<c->n_blocks, kTile, 0, c->stream>>>(P);
   }
@@ -625,6 +648,7 @@ void enqueue_update(cbm_ctx* c, const Params<T>& P, bool after_kernel = false) {
   }
   ScanArgs A{c->cell_count, c->cell_start, c->scan_state, c->n_cells, c->n_scan_tiles, c->ctr,
              resort_flag(c)};
+  A.crowd = may_be_sparse(c->cfg);
   if (P.hist_in_de) {
     A.due = nullptr;
     A.commit = 1;
@@ -668,9 +692,10 @@ int kernels_per_step(const cbm_ctx* c) {
   if (rule_needed(k)) n += 1;           // rule (with births and deaths when fate is on)
   if (k.fate != CBM_FATE_NONE) n += 1;  // compaction
   n += 1;                               // agent DE
-  if (c->tile_blocks && k.neighbors == CBM_NEIGH_CLVD) n += 1;  // its steps on the list
-  if (c->pos32) n += 1;                 // its Float32 positions (Float64 3D walks)
-  if (c->pos_rows) n += 1;              // its position rows (Float32 3D walks)
+  const bool tiled = c->tile_blocks && !c->sparse;
+  if (tiled && k.neighbors == CBM_NEIGH_CLVD) n += 1;  // its steps on the list
+  if (c->pos32 && !tiled) n += 1;       // its Float32 positions (Float64 walks by threads)
+  if (c->pos_rows && !tiled) n += 1;    // its position rows (Float32 walks by threads)
   if (k.medium) n += 1;
   n += hist_in_de(k) ? 3 : 4;           // sort hist, scan, scatter, place
   if (k.neighbors == CBM_NEIGH_VERLET_DISPLACEMENT) n += 1;
@@ -872,6 +897,7 @@ struct FirstSort {  // the re-sort half of update!, for loadToPlatform!
     k_sort_hist<T, D><<<c->n_blocks, kTile, 0, c->stream>>>(P, 0);
     ScanArgs A{c->cell_count, c->cell_start, c->scan_state, c->n_cells, c->n_scan_tiles, c->ctr,
                resort_flag(c)};
+    A.crowd = may_be_sparse(c->cfg);
     k_scan_cells<<<c->n_scan_tiles, kTile, 0, c->stream>>>(A);
     k_sort_scatter<T><<<c->n_blocks, kTile, 0, c->stream>>>(P);
     k_sort_place<T, D><<<c->n_blocks, kTile, 0, c->stream>>>(P);
@@ -898,17 +924,21 @@ void* dalloc(cbm_ctx* c, size_t bytes, bool* ok) {
   return p;
 }
 
+void drop_graphs(cbm_ctx* c) {
+  for (int q = 0; q < 2; ++q)
+    for (cudaGraphExec_t* g : {&c->graph[q], &c->tgraph[q], &c->chain[q]}) {
+      if (*g) cudaGraphExecDestroy(*g);
+      *g = nullptr;
+    }
+}
+
 void free_all(cbm_ctx* c) {
   for (auto& m : c->marks) {
     cudaEventDestroy(m.ev[0]);
     cudaEventDestroy(m.ev[1]);
   }
   c->marks.clear();
-  for (int q = 0; q < 2; ++q) {
-    if (c->graph[q]) cudaGraphExecDestroy(c->graph[q]);
-    if (c->tgraph[q]) cudaGraphExecDestroy(c->tgraph[q]);
-    if (c->chain[q]) cudaGraphExecDestroy(c->chain[q]);
-  }
+  drop_graphs(c);
   for (int q = 0; q < 2; ++q) {
     for (auto& m : c->gmarks[q]) {
       cudaEventDestroy(m.ev[0]);
@@ -938,12 +968,19 @@ int flags_to_status(int err) {
   return CBM_OK;
 }
 
-// the counters after all that is enqueued: one copy to page-locked memory and
-// one wait
+// The counters after all that is enqueued: one copy to page-locked memory and
+// one wait.  With them comes the choice of the walk for the steps to come (the
+// sums are the same bits either way); steps being timed keep theirs.
 int read_counters(cbm_ctx* c, Counters* h) {
   CUDA_TRY(c, cudaMemcpyAsync(c->h_ctr, c->ctr, sizeof(Counters), cudaMemcpyDeviceToHost, c->stream));
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   *h = *c->h_ctr;
+  const long long n = h->N[c->parity];
+  if (c->tile_blocks && c->pair_list && n > 0 && !c->graph_timing) {
+    const bool sparse = is_sparse(c->cfg, (double)h->crowd / (double)n, n, c->sparse);
+    if (sparse != c->sparse) drop_graphs(c);
+    c->sparse = sparse;
+  }
   return CBM_OK;
 }
 
@@ -1137,11 +1174,12 @@ int cbm_create(cbm_ctx** out, const cbm_config* cfg) {
       const long long tiles = (long long)(n + 31) / 32, warps = (long long)c->n_sm * bps;
       c->tile_blocks = (int)(warps < tiles ? warps : tiles);
     }
-    if (walk_by_thread(k))
+    const bool threads = walk_by_thread(k) || may_be_sparse(k);
+    if (threads)
       c->pair_list = dalloc(c, (size_t)c->de_blocks * kTile * kPairCap4 * sizeof(int4), &ok);
     // the filter's copies of the committed positions (a walk of reflected
     // positions reads those)
-    const bool copies = walk_by_thread(k) && k.walls != CBM_WALLS_REFLECT;
+    const bool copies = threads && k.walls != CBM_WALLS_REFLECT;
     if (copies && c->tsize == 8) c->pos32 = dalloc(c, n * sizeof(float4), &ok);
     if (copies && c->tsize == 4) {
       c->rows_stride = (int)((n + 3) & ~(size_t)3);  // rows start on 16 bytes

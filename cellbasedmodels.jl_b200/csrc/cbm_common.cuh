@@ -85,6 +85,7 @@ struct Counters {
   unsigned de_ticket;   // tile tickets of the force kernel (reset by its last block)
   unsigned de_done;     // blocks of the force kernel that have finished
   unsigned hist_done;   // blocks of the sort's histogram that have finished
+  unsigned long long crowd;  // squares of the cells' counts, summed by the last scan (if asked)
 };
 
 // The commit of update!: the next parity's counters from those of parity p.
@@ -316,6 +317,7 @@ struct ScanArgs {
   // the scan also commits the counters of a step of parity p that always
   // re-sorts, whose force kernel made the histogram
   int commit = 0;
+  int crowd = 0;                   // add the squares of the counts to the counters' crowd
   int parity = 0;
   double dt = 0.0;
 };
@@ -366,6 +368,14 @@ static __global__ void __launch_bounds__(kTile) k_scan_cells(ScanArgs A) {
   for (int k = 0; k < kScanItems; ++k) {
     vals[k] = s_cells[scan_pad(first + k)];
     sum += vals[k];
+  }
+  if (A.crowd) {
+    unsigned long long sq = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) sq += (unsigned long long)vals[k] * (unsigned)vals[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(kFull, sq, o);
+    if ((threadIdx.x & 31) == 0 && sq) atomicAdd(&C->crowd, sq);
   }
   int total;
   int ex = block_exscan(sum, warp_sums, &total);

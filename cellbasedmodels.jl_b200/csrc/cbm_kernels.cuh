@@ -65,7 +65,7 @@ struct Params {
   V4* KOUT;
   int no_prune;
   int hist_in_de;       // the force kernel makes the histogram of the re-sort
-  int tiled;            // k_agent_de_tile takes the 3D cell walks of this configuration
+  int tiled;            // k_agent_de_tile takes the 3D cell walks
   V4* POLD;             // positions at the last Verlet rebuild (slot order)
   int* inv;             // agent index -> slot of A
   int* cell_of_slot;    // cell of each A slot
@@ -1628,8 +1628,8 @@ __device__ __forceinline__ bool clvd_walks_cells(const Params<T>& P) {
   return P.ctr->events != 0 && !P.ctr->list_valid && P.force_in_list;
 }
 
-// Slot s of N; `list` is this thread's partner list (null: none); `live`
-// holds the lanes of this warp whose slot is below N.
+// Slot s of N; `list` is this thread's partner list (a 3D walk of the cells
+// needs one); `live` holds the lanes of this warp whose slot is below N.
 template <typename T, int D>
 __device__ __forceinline__ void agent_de(const Params<T>& P, const int N, const int s,
                                          int4* const list, const unsigned live) {
@@ -2626,6 +2626,7 @@ __global__ void __launch_bounds__(kTile) k_sort_hist(Params<T> P, int commit) {
     if (s == 0) {
       C->scan_ticket = 0u;  // fresh tickets and tile-state generation for the scan
       C->scan_epoch = C->scan_epoch + 1u;
+      C->crowd = 0ull;
     }
     int c = -1;
     if (s < slots && P.IB[s] >= 0) {
