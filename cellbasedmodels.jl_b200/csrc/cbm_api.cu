@@ -805,12 +805,28 @@ struct DEOccupancy {
   }
 };
 
-// resident one-warp blocks of the tiled force walk per multiprocessor
+// Resident one-warp blocks of the tiled force walk per multiprocessor.  Its
+// preferred split between shared memory and L1 holds for what runs beside it:
+// an SM takes no block of another split until it is idle.  In Float64 the
+// field's kernels have blocks on every SM, and the walk waited for them (80^3
+// nodes with 6144 agents 48.8 us a step, 37.0 with the split shared; 128^3
+// with 6291 58.3 and 47.2).  In Float32 they leave SMs free, and the stencils
+// of 256^3 nodes lose 1.5 % with less L1.
 template <typename T, int D>
 struct TileOccupancy {
-  static void run(cbm_ctx*, int* bps) {
-    cudaFuncSetAttribute(k_agent_de_tile<T>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         kTileCarveout);
+  static void run(cbm_ctx* c, int* bps) {
+    auto prefer = [](auto* kernel) {
+      cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, kTileCarveout);
+    };
+    prefer(k_agent_de_tile<T>);
+    if constexpr (D == 3 && sizeof(T) == 8) {
+      if (c->cfg.medium) {
+        prefer(k_medium_grad_3d_vec<T>);
+        prefer(k_medium_de_3d_vec<T>);
+        prefer(k_medium_links<T, D>);
+        prefer(k_medium_apply<T, D>);
+      }
+    }
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_agent_de_tile<T>, 32, 0) !=
             cudaSuccess ||
         *bps < 1)
