@@ -103,6 +103,7 @@ struct cbm_ctx {
   int n_blocks = 0;
   int n_sm = 148;             // multiprocessors of the device (grid of the compaction)
   int de_blocks = 1;          // persistent grid of the force kernel
+  int split = -1;             // preferred percentage of shared memory of the step's kernels
   int tile_blocks = 0;        // resident blocks of k_agent_de_tile (0: not used)
   bool sparse = false;        // the walks that the tiles could take are made by threads
   void* pair_list = nullptr;  // partner lists of the walks by threads
@@ -211,10 +212,31 @@ struct Prof {
 // launches, and the kernel's pdl_wait() orders its memory accesses after
 // it.  A plain launch while kernels are timed (the event records sit
 // between).
+//
+// Beside a 3D medium every kernel asks for the same split of an SM between
+// shared memory and L1: the two pipelines run at once, and an SM takes no
+// block of a kernel with another split until it is idle.  Left to themselves
+// the vector stencils prefer L1 and the force kernels and the scan shared
+// memory, and each waited for the other's blocks to leave.  The tiled walk's
+// split suits them; beside a walk by threads it is what three of its blocks
+// need (164 KB; 3e5 agents on 160^3 nodes, Float64, 745 us a step, with the
+// tiles' 132 KB and two blocks 776).  Us a step before / so / with stencils
+// that staged planes in shared memory, which had no such conflict:
+//   no neighbors, uptake and chemotaxis by atomics, Float32
+//     1e4 agents, 100^3 nodes 45 / 26 / 32;  4e4, 160^3 77 / 57 / 63
+//   CellLinked, the same exchange in order, Float64
+//     4479 agents, 72^3 44 / 36 / 38;  10616, 96^3 51 / 40 / 44
+//   CellLinked, Float32, 2e5 agents, 256^3 180 / 182 / 246
+constexpr int kThreadCarveout = 72;
 template <typename... KP, typename... A>
 void launch_pdl(cbm_ctx* c, bool pdl, void (*kern)(KP...), dim3 grid, dim3 block, size_t smem,
                 A&&... args) {
-  launch_serial(c->stream, pdl && !c->prof, kern, grid, block, smem, std::forward<A>(args)...);
+  launch_split(c->stream, c->split, pdl && !c->prof, kern, grid, block, smem,
+               std::forward<A>(args)...);
+}
+template <typename... KP, typename... A>
+void launch(cbm_ctx* c, void (*kern)(KP...), unsigned grid, unsigned block, A&&... args) {
+  launch_pdl(c, false, kern, dim3(grid), dim3(block), 0, std::forward<A>(args)...);
 }
 
 // r^2 (1 + 1e-5) rounded up to T: a squared distance at or above it has a
@@ -495,7 +517,7 @@ void enqueue_medium_rule(cbm_ctx* c, const Params<T>& P) {
       k_medium_grad_2d<T><<<stencil_grid(c), dim3(kStX, kStY), 0, c->stream>>>(P);
     else if (D == 3)
       if (vec_medium(c))
-        k_medium_grad_3d_vec<T><<<vec_grid(c), kTile, 0, c->stream>>>(P, vec_z_run(c));
+        launch_pdl(c, false, k_medium_grad_3d_vec<T>, vec_grid(c), dim3(kTile), 0, P, vec_z_run(c));
       else
         k_medium_grad_3d<T><<<stencil_grid_3d(c), dim3(kStX, kStY), 0, c->stream>>>(P, stencil_z_run(c));
     else
@@ -511,12 +533,12 @@ template <typename T, int D>
 void enqueue_links(cbm_ctx* c, const Params<T>& P) {
   cudaMemsetAsync(c->link_head, 0xff, link_head_bytes(c), c->stream);
   PROF("k_medium_links");
-  k_medium_links<T, D><<<grid_blocks(c->cfg.n_max << D), kTile, 0, c->stream>>>(P);
+  launch(c, k_medium_links<T, D>, grid_blocks(c->cfg.n_max << D), kTile, P);
 }
 template <typename T, int D>
 void enqueue_apply(cbm_ctx* c, const Params<T>& P) {
   PROF("k_medium_apply");
-  k_medium_apply<T, D><<<grid_blocks(c->cfg.n_max << D), kTile, 0, c->stream>>>(P);
+  launch(c, k_medium_apply<T, D>, grid_blocks(c->cfg.n_max << D), kTile, P);
 }
 template <typename T, int D>
 void enqueue_gather(cbm_ctx* c, const Params<T>& P) {
@@ -527,7 +549,7 @@ void enqueue_gather(cbm_ctx* c, const Params<T>& P) {
   constexpr int W = GatherPatch<D>::kWarps;
   const dim3 grid((unsigned)((nm[0] + 31) / 32), (unsigned)((py + W - 1) / W),
                   (unsigned)((nm[2] + GatherPatch<D>::kZ - 1) / GatherPatch<D>::kZ));
-  k_secrete_rows<T, D><<<grid, W * 32, 0, c->stream>>>(P);
+  launch_pdl(c, false, k_secrete_rows<T, D>, grid, dim3(W * 32), 0, P);
 }
 // walls, births and deaths, and the exchange that atomics add
 template <typename T, int D>
@@ -535,15 +557,15 @@ void enqueue_rule(cbm_ctx* c, const Params<T>& P) {
   const cbm_config& k = c->cfg;
   if (needs_snapshot(k)) {
     PROF("k_medium_snapshot");
-    k_medium_snapshot<T><<<grid_blocks(c->n_nodes), kTile, 0, c->stream>>>(P);
+    launch(c, k_medium_snapshot<T>, grid_blocks(c->n_nodes), kTile, P);
   }
   if (!rule_needed(k)) return;
   if (k.fate != CBM_FATE_NONE) {
     PROF("k_agent_fate");
-    k_agent_fate<T, D><<<fate_tiles(c->cfg.n_max), kTile, 0, c->stream>>>(P);
+    launch(c, k_agent_fate<T, D>, fate_tiles(c->cfg.n_max), kTile, P);
   } else {
     PROF("k_agent_rule");
-    k_agent_rule<T, D><<<c->n_blocks, kTile, 0, c->stream>>>(P);
+    launch(c, k_agent_rule<T, D>, c->n_blocks, kTile, P);
   }
 }
 template <typename T, int D>
@@ -563,11 +585,11 @@ void enqueue_agent_de(cbm_ctx* c, const Params<T>& P) {
   const int integ = c->cfg.integrator;
   if (P.PA32) {
     PROF("k_pos32");
-    k_pos32<T><<<c->n_blocks, kTile, 0, c->stream>>>(P);
+    launch(c, k_pos32<T>, c->n_blocks, kTile, P);
   }
   if (P.PS) {
     PROF("k_pos_rows");
-    k_pos_rows<T><<<c->n_blocks, kTile, 0, c->stream>>>(P);
+    launch(c, k_pos_rows<T>, c->n_blocks, kTile, P);
   }
   if (integ != CBM_INT_HEUN && integ != CBM_INT_RK4 && integ != CBM_INT_EULER_HEUN) {
     if constexpr (D == 3) {
@@ -592,10 +614,10 @@ void enqueue_agent_de(cbm_ctx* c, const Params<T>& P) {
     }
     {
       PROF("k_agent_de");
-      k_agent_de<T, D><<<grid, kTile, 0, c->stream>>>(Q);
+      launch(c, k_agent_de<T, D>, grid, kTile, Q);
     }
     PROF("k_stage_combine");
-    k_stage_combine<T, D><<<c->n_blocks, kTile, 0, c->stream>>>(P, op);
+    launch(c, k_stage_combine<T, D>, c->n_blocks, kTile, P, op);
   };
   if (integ == CBM_INT_HEUN) {
     stage(false, kHeunStage);
@@ -619,7 +641,7 @@ void enqueue_medium_de(cbm_ctx* c, const Params<T>& P) {
       k_medium_de_2d<T><<<stencil_grid(c), dim3(kStX, kStY), 0, c->stream>>>(P);
     else if (D == 3)
       if (vec_medium(c))
-        k_medium_de_3d_vec<T><<<vec_grid(c), kTile, 0, c->stream>>>(P, vec_z_run(c));
+        launch_pdl(c, false, k_medium_de_3d_vec<T>, vec_grid(c), dim3(kTile), 0, P, vec_z_run(c));
       else
         k_medium_de_3d<T><<<stencil_grid_3d(c), dim3(kStX, kStY), 0, c->stream>>>(P, stencil_z_run(c));
     else
@@ -643,7 +665,7 @@ template <typename T, int D>
 void enqueue_update(cbm_ctx* c, const Params<T>& P, bool after_kernel = false) {
   if (c->cfg.fate != CBM_FATE_NONE) {
     PROF("k_compact");
-    k_compact<T, D><<<c->n_sm, kCompactThreads, 0, c->stream>>>(P);
+    launch(c, k_compact<T, D>, c->n_sm, kCompactThreads, P);
     after_kernel = true;
   }
   ScanArgs A{c->cell_count, c->cell_start, c->scan_state, c->n_cells, c->n_scan_tiles, c->ctr,
@@ -679,7 +701,7 @@ template <typename T, int D>
 void enqueue_neighbors(cbm_ctx* c, const Params<T>& Q) {
   if (c->cfg.neighbors == CBM_NEIGH_VERLET_DISPLACEMENT) {
     PROF("k_verlet_list");
-    k_verlet_list<T, D><<<c->n_blocks, kTile, 0, c->stream>>>(Q, 1);
+    launch(c, k_verlet_list<T, D>, c->n_blocks, kTile, Q, 1);
   }
 }
 
@@ -805,28 +827,12 @@ struct DEOccupancy {
   }
 };
 
-// Resident one-warp blocks of the tiled force walk per multiprocessor.  Its
-// preferred split between shared memory and L1 holds for what runs beside it:
-// an SM takes no block of another split until it is idle.  In Float64 the
-// field's kernels have blocks on every SM, and the walk waited for them (80^3
-// nodes with 6144 agents 48.8 us a step, 37.0 with the split shared; 128^3
-// with 6291 58.3 and 47.2).  In Float32 they leave SMs free, and the stencils
-// of 256^3 nodes lose 1.5 % with less L1.
+// resident one-warp blocks of the tiled force walk per multiprocessor
 template <typename T, int D>
 struct TileOccupancy {
-  static void run(cbm_ctx* c, int* bps) {
-    auto prefer = [](auto* kernel) {
-      cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, kTileCarveout);
-    };
-    prefer(k_agent_de_tile<T>);
-    if constexpr (D == 3 && sizeof(T) == 8) {
-      if (c->cfg.medium) {
-        prefer(k_medium_grad_3d_vec<T>);
-        prefer(k_medium_de_3d_vec<T>);
-        prefer(k_medium_links<T, D>);
-        prefer(k_medium_apply<T, D>);
-      }
-    }
+  static void run(cbm_ctx*, int* bps) {
+    cudaFuncSetAttribute(k_agent_de_tile<T>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                         kTileCarveout);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_agent_de_tile<T>, 32, 0) !=
             cudaSuccess ||
         *bps < 1)
@@ -1211,6 +1217,7 @@ int cbm_create(cbm_ctx** out, const cbm_config* cfg) {
       c->c[q] = dalloc(c, (size_t)c->n_nodes * S, &ok);
       for (int d = 0; d < 3; ++d) c->grad[q][d] = dalloc(c, (size_t)c->n_nodes * S, &ok);
     }
+    if (k.dims == 3 && vec_medium(c)) c->split = walk_by_thread(k) ? kThreadCarveout : kTileCarveout;
     if (orders_exchange(k)) {
       size_t nb = 0;
       for (int d = 0; d < k.dims; ++d) nb += 2 * (size_t)k.n_medium[d];

@@ -37,20 +37,31 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // serialization when `pdl` (then the operation before it on st must be a
 // kernel launch, and kern calls pdl_wait() before its first global access).
 // Errors are seen like those of <<<>>> launches, by cudaGetLastError.
+// split: the preferred percentage of shared memory, -1 for the kernel's own.
 template <typename... KP, typename... A>
-inline void launch_serial(cudaStream_t st, bool pdl, void (*kern)(KP...), dim3 grid, dim3 block,
-                          size_t smem, A&&... args) {
+inline void launch_split(cudaStream_t st, int split, bool pdl, void (*kern)(KP...), dim3 grid,
+                         dim3 block, size_t smem, A&&... args) {
   cudaLaunchConfig_t lc = {};
   lc.gridDim = grid;
   lc.blockDim = block;
   lc.dynamicSmemBytes = smem;
   lc.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute at[2];
   lc.attrs = at;
-  lc.numAttrs = pdl ? 1 : 0;
+  if (pdl) {
+    at[lc.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[lc.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (split >= 0) {
+    at[lc.numAttrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at[lc.numAttrs++].val.sharedMemCarveout = (unsigned)split;
+  }
   cudaLaunchKernelEx(&lc, kern, std::forward<A>(args)...);
+}
+template <typename... KP, typename... A>
+inline void launch_serial(cudaStream_t st, bool pdl, void (*kern)(KP...), dim3 grid, dim3 block,
+                          size_t smem, A&&... args) {
+  launch_split(st, -1, pdl, kern, grid, block, smem, std::forward<A>(args)...);
 }
 
 // device error bits (cbm_sync reports the first as a status code)
