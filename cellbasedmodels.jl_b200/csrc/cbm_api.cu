@@ -409,6 +409,16 @@ bool orders_exchange(const cbm_config& k) {
   return exchanges(k) && k.medium_sampling == CBM_MEDIUM_BILINEAR &&
          k.neighbors == CBM_NEIGH_CELL_LINKED;
 }
+// the exchange in agent order by lists: an entry per agent and stencil node
+unsigned long long list_entries(const cbm_config& k) {
+  return (unsigned long long)(k.n_max > 0 ? k.n_max : 1) << k.dims;
+}
+bool exchange_by_lists(const cbm_config& k) {
+  if (!orders_exchange(k)) return false;
+  unsigned long long nodes = 1;
+  for (int d = 0; d < k.dims; ++d) nodes *= (unsigned long long)k.n_medium[d];
+  return list_entries(k) * kListNodes <= nodes;
+}
 bool rule_needed(const cbm_config& k) {
   return k.walls == CBM_WALLS_REFLECT || (exchanges(k) && !orders_exchange(k)) ||
          k.fate != CBM_FATE_NONE;
@@ -946,6 +956,12 @@ void* dalloc(cbm_ctx* c, size_t bytes, bool* ok) {
   return p;
 }
 
+// the nodes of a step with lists keep the priorities of the streams they were
+// captured on
+unsigned instantiate_flags(const cbm_ctx* c) {
+  return c->link_buckets ? cudaGraphInstantiateFlagUseNodePriority : 0;
+}
+
 void drop_graphs(cbm_ctx* c) {
   for (int q = 0; q < 2; ++q)
     for (cudaGraphExec_t* g : {&c->graph[q], &c->tgraph[q], &c->chain[q]}) {
@@ -1098,7 +1114,15 @@ int cbm_create(cbm_ctx** out, const cbm_config* cfg) {
     return rc;
   }
   if (k.medium) {
-    se = cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking);
+    // Where the exchange is by lists the agents' kernels, which nothing of the
+    // field's delays for long, go first (2e5 agents on 256^3 nodes 180 us a
+    // step without, 175 with); the gather is on the field's side, and waits
+    // for it would then grow (2D, 2e5 agents on 1024^2: 54.7 without, 58.8).
+    int least = 0, greatest = 0;
+    se = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+    if (se == cudaSuccess)
+      se = cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking,
+                                        exchange_by_lists(k) ? greatest : least);
     for (cudaEvent_t* e :
          {&c->fork_ev, &c->join_ev, &c->links_ev, &c->field_ev, &c->de_ev, &c->update_ev})
       if (se == cudaSuccess) se = cudaEventCreateWithFlags(e, cudaEventDisableTiming);
@@ -1223,9 +1247,8 @@ int cbm_create(cbm_ctx** out, const cbm_config* cfg) {
       for (int d = 0; d < k.dims; ++d) nb += 2 * (size_t)k.n_medium[d];
       c->gather_box = (int*)dalloc(c, nb * 4, &ok);
     }
-    // an entry per agent and stencil node
-    const unsigned long long ne = (unsigned long long)n << k.dims;
-    if (orders_exchange(k) && ne * kListNodes <= (unsigned long long)c->n_nodes) {
+    if (exchange_by_lists(k)) {
+      const unsigned long long ne = list_entries(k);
       c->link_buckets = 1024;
       while (c->link_buckets < ne) c->link_buckets *= 2;
       c->link_head = (unsigned*)dalloc(c, link_head_bytes(c), &ok);
@@ -1588,7 +1611,7 @@ int cbm_step(cbm_ctx* c, int32_t nsteps, int32_t flags) {
         dispatch<ChainSteps>(c, p);
         cudaError_t e = cudaStreamEndCapture(c->stream, &g);
         if (e != cudaSuccess) return fail(c, CBM_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
-        e = cudaGraphInstantiate(&c->chain[p], g, 0);
+        e = cudaGraphInstantiate(&c->chain[p], g, instantiate_flags(c));
         cudaGraphDestroy(g);
         if (e != cudaSuccess) return fail(c, CBM_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(e));
       }
@@ -1613,7 +1636,7 @@ int cbm_step(cbm_ctx* c, int32_t nsteps, int32_t flags) {
         c->prof_used = nullptr;
         cudaError_t e = cudaStreamEndCapture(c->stream, &g);
         if (e != cudaSuccess) return fail(c, CBM_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
-        e = cudaGraphInstantiate(&graphs[p], g, 0);
+        e = cudaGraphInstantiate(&graphs[p], g, instantiate_flags(c));
         cudaGraphDestroy(g);
         if (e != cudaSuccess) return fail(c, CBM_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(e));
       }
