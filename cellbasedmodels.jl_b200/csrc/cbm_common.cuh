@@ -99,7 +99,9 @@ struct Counters {
   unsigned long long crowd;  // squares of the cells' counts, summed by the last scan (if asked)
 };
 
-// The commit of update!: the next parity's counters from those of parity p.
+// The commit of update!: the next parity's counters from those of parity p (N
+// <- N + NAdd - NRemove, t += dt, step += 1: update.jl:201-298), and the
+// re-sort decision of computeNeighbors!.
 // One thread of one kernel of the step does it, once no other thread still
 // reads the step's births, deaths and flag.
 __device__ __forceinline__ void commit_counters(Counters* C, int p, double dt, bool resort) {

@@ -2580,8 +2580,6 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact(Params<T> P) {
   }
 }
 
-// N <- N + NAdd - NRemove, t += dt, step += 1 (update.jl:201-298), and the
-// re-sort decision of computeNeighbors!.  One thread.
 // ---------------------------------------------------------------------------
 // End of step: B -> A.  Without a re-sort the working slots are copied; with
 // one, live working slots are counting-sorted by (cell, agent index) into A
