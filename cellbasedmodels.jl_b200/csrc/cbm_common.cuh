@@ -164,7 +164,7 @@ __device__ __forceinline__ int floordiv(float a, float b) {
 //    [1, 4), and these are compared at every exponent.
 //  - inv is within 3.5 u of 1 / b, so y is 1 / b less at most (3.5 u)^2 of it,
 //    rounded: the rounded reciprocal unless a midpoint lies in between, at
-//    k u^2 / 2 from 1 / b with a whole k <= 12.  The quotient needs no more
+//    k u^2 / b from 1 / b with a whole k <= 12.  The quotient needs no more
 //    than |b y - 1| b < 2 u (1 - u) for b in [1, 2), since a - b m is a
 //    multiple of u times the spacing for every midpoint m; a y that is not the
 //    rounded one keeps to that too, unless b >= 2 - 12 u.  There the k of the
